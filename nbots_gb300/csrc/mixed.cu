@@ -39,6 +39,7 @@
 #include <new>
 #include <vector>
 
+#include "allreduce.cuh"
 #include "perm.cuh"
 #include "persist.cuh"
 
@@ -181,8 +182,15 @@ struct MixScalars {
         }
         return upd;
     }
-    // A reliable update's {|r|^2, r.z} (FP64): 2 stop, else 0 with beta.
-    __device__ __forceinline__ int replaced(const double (&t)[2], uint32_t max_iter, FF& beta) {
+    // A reliable update's {|r|^2, r.z, r.p} (FP64), r the recomputed residual
+    // and p the last direction: 2 stop, else 0 with beta.  The recursive
+    // residual was orthogonal to p, the recomputed one is only up to the
+    // rounding of b - A u, so the next step's numerator is r.(z + beta p), not
+    // r.z: near the FP64 floor of a system the difference is no longer small,
+    // and with r.z the error stayed in every later step until the iteration
+    // diverged (the 20,000-point T3 L-shape at relres 8e-12: 36 after 40,000
+    // iterations).
+    __device__ __forceinline__ int replaced(const double (&t)[3], uint32_t max_iter, FF& beta) {
         rr64 = t[0];
         rmax2 = (float)rr64;
         nupd++;
@@ -191,7 +199,13 @@ struct MixScalars {
         if (!stop) {
             const FF rzn = ff_from_double(t[1]);
             beta = ff_div(rzn, rz);
-            rz = rzn;
+            const FF rp = ff_add(rzn, ff_mul(beta, ff_from_double(t[2])));
+            if (rp.hi > 0.1f * rzn.hi) {
+                rz = rp;
+            } else {  // p points uphill: start again from z
+                beta = FF{0.f, 0.f};
+                rz = rzn;
+            }
         }
         return stop ? 2 : 0;
     }
@@ -282,13 +296,18 @@ __device__ __forceinline__ Own own_vectors(const MixArgs& a, unsigned char* smem
     return o;
 }
 
+// rp + r.p of one node row, p float-float
+__device__ __forceinline__ double dot_with(double r0, double r1, float4 p, double rp) {
+    return fma(r0, (double)p.x + (double)p.z, fma(r1, (double)p.y + (double)p.w, rp));
+}
+
 // r = b - A u in FP64 for the own rows, stored as float-float; z = r / Aii
-// (float-float); accumulates |r|^2 (FP64), r.z and optionally |b|^2; with
-// set_p, p = z (own copy and the global one).
+// (float-float); accumulates |r|^2 (FP64), r.z and optionally |b|^2 and r.p;
+// with set_p, p = z (own copy and the global one).
 template <int kThreads>
 __device__ __forceinline__ void true_residual(const MixArgs& a, const Own& o, uint32_t s0,
                                               uint32_t s1, double& rr, FFAcc& rz, double* bb,
-                                              bool set_p) {
+                                              double* rp, bool set_p) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t nw = kThreads / 32;
     const double2* __restrict__ u = reinterpret_cast<const double2*>(a.u);
@@ -301,6 +320,7 @@ __device__ __forceinline__ void true_residual(const MixArgs& a, const Own& o, ui
         const double r0 = bi.x - au.x, r1 = bi.y - au.y;
         rr = fma(r0, r0, fma(r1, r1, rr));
         if (bb) *bb = fma(bi.x, bi.x, fma(bi.y, bi.y, *bb));
+        if (rp) *rp = dot_with(r0, r1, o.p[li], *rp);
         const FF f0 = ff_from_double(r0), f1 = ff_from_double(r1);
         o.r[li] = make_float4(f0.hi, f1.hi, f0.lo, f1.lo);
         const float2 di = o.dv[li];
@@ -358,7 +378,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
         __syncwarp();
         double rrl = 0.0, bbl = 0.0;
         FFAcc rzk{0.f, 0.f};
-        true_residual<kThreads>(a, o, s0, s1, rrl, rzk, &bbl, true);
+        true_residual<kThreads>(a, o, s0, s1, rrl, rzk, &bbl, nullptr, true);
         const FF t = rzk.result();
         double v[3] = {rrl, bbl, (double)t.hi + (double)t.lo};
         group_publish<3>(v, red, part2, rank);
@@ -456,15 +476,15 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
                 o.x[li] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
             if (sync()) goto done;
-            double rrl = 0.0;
+            double rrl = 0.0, rpl = 0.0;
             FFAcc rzk{0.f, 0.f};
-            true_residual<kThreads>(a, o, s0, s1, rrl, rzk, nullptr, false);
+            true_residual<kThreads>(a, o, s0, s1, rrl, rzk, nullptr, &rpl, false);
             const FF t = rzk.result();
-            double v[2] = {rrl, (double)t.hi + (double)t.lo};
-            group_publish<2>(v, red, part2, rank);
+            double v[3] = {rrl, (double)t.hi + (double)t.lo, rpl};
+            group_publish<3>(v, red, part2, rank);
             if (sync()) goto done;
-            double tt[2];
-            group_reduce0<2>(part2, G, tt);
+            double tt[3];
+            group_reduce0<3>(part2, G, tt);
             if (threadIdx.x == 0) {
                 FF be;
                 s_flag = sc.replaced(tt, a.max_iter, be);
@@ -558,9 +578,13 @@ uint32_t keep_permille(const nbg_bsr_t& A, double bytes_per_entry = 32.0) {
     return (uint32_t)(1000.0 * budget / stream);
 }
 
+// Vectors, partial sums, then what a launch needs at zero: barrier, status
+// and result words and the records and words of the slice form's sums.
+constexpr size_t kMixTail = 3 * 256 + kArBytes + 2 * kExactBytes;
+
 size_t mixed_core_bytes(uint32_t N) {
     const size_t f = align256((size_t)N * 4), h = align256((size_t)N * 4);
-    return 6 * f + 2 * h + align256(kMaxBlocks * 6 * 8) + 3 * 256;
+    return 6 * f + 2 * h + align256(kMaxBlocks * 6 * 8) + kMixTail;
 }
 
 // The vector slots at the start of a workspace (indexed by node row, a
@@ -630,7 +654,7 @@ constexpr uint32_t kGhostKeys = 32768;  // outside-column references per block t
 struct GhostArgs {
     const uint16_t* lcol;   // local column of every layout entry
     const uint32_t* ids;    // kGhostMax ghost node ids per block, ascending
-    const uint32_t* count;  // ghosts per block
+    const uint32_t* count;  // ghosts per block, then the block's widest slice
     uint32_t scap;          // own row slots of the largest block
     uint32_t pcap;          // row slots + ghosts, largest over the blocks
     uint32_t gcap;          // ghosts, largest over the blocks
@@ -648,15 +672,17 @@ __global__ void __launch_bounds__(1024, 1) k_ghost_plan(nbg_bsr_t A, uint16_t* l
     extern __shared__ __align__(16) uint32_t keys[];  // kGhostKeys
     __shared__ uint32_t s_n;
     __shared__ uint32_t s_scan[32];
+    __shared__ uint32_t s_wide;  // widest slice
     const uint32_t tid = threadIdx.x, bd = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t nw = bd >> 5;
     uint32_t s0, s1;
     slice_range(A.n_slices, s0, s1);
     const uint32_t n0 = s0 * 32, nslot = (s1 - s0) * 32;
-    if (tid == 0) s_n = 0;
+    if (tid == 0) s_n = s_wide = 0;
     __syncthreads();
     for (uint32_t s = s0 + warp; s < s1; s += nw) {
         const uint32_t i = s * 32 + lane;
+        if (lane == 0) atomicMax(&s_wide, A.slice_off[s + 1] - A.slice_off[s]);
         if (i >= A.Nn) continue;
         for (uint32_t k = A.slice_off[s]; k < A.slice_off[s + 1]; k++) {
             const uint32_t c = A.bcol[(size_t)k * 32 + lane];
@@ -724,7 +750,10 @@ __global__ void __launch_bounds__(1024, 1) k_ghost_plan(nbg_bsr_t A, uint16_t* l
         if (j == 0 || keys[j] != keys[j - 1]) my[pos++] = keys[j];
     __syncthreads();
     for (uint32_t j = tid; j < u; j += bd) keys[j] = my[j];
-    if (tid == 0) count[blockIdx.x] = u;
+    if (tid == 0) {
+        count[blockIdx.x] = u;
+        count[gridDim.x + blockIdx.x] = s_wide;
+    }
     __syncthreads();
     for (uint32_t s = s0 + warp; s < s1; s += nw) {
         const uint32_t i = s * 32 + lane;
@@ -793,7 +822,8 @@ __device__ __forceinline__ float4* ghost_x(const MixArgs& a) { return a.x4; }
 template <int kThreads>
 __device__ __forceinline__ void true_residual_ghost(const MixArgs& a, float4* P,
                                                     uint32_t s0, uint32_t s1, double& rr,
-                                                    FFAcc& rz, double* bb, bool set_p) {
+                                                    FFAcc& rz, double* bb, double* rp,
+                                                    bool set_p) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t nw = kThreads / 32;
     const double2* __restrict__ u = reinterpret_cast<const double2*>(a.u);
@@ -808,6 +838,7 @@ __device__ __forceinline__ void true_residual_ghost(const MixArgs& a, float4* P,
         const double r0 = bi.x - au.x, r1 = bi.y - au.y;
         rr = fma(r0, r0, fma(r1, r1, rr));
         if (bb) *bb = fma(bi.x, bi.x, fma(bi.y, bi.y, *bb));
+        if (rp) *rp = dot_with(r0, r1, P[li], *rp);
         const FF f0 = ff_from_double(r0), f1 = ff_from_double(r1);
         r4[i] = make_float4(f0.hi, f1.hi, f0.lo, f1.lo);
         const float2 di = dinv[i];
@@ -865,7 +896,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
         }
         double rrl = 0.0, bbl = 0.0;
         FFAcc rzk{0.f, 0.f};
-        true_residual_ghost<kThreads>(a, P, s0, s1, rrl, rzk, &bbl, true);
+        true_residual_ghost<kThreads>(a, P, s0, s1, rrl, rzk, &bbl, nullptr, true);
         const FF t = rzk.result();
         double v[3] = {rrl, bbl, (double)t.hi + (double)t.lo};
         group_publish<3>(v, red, part2, rank);
@@ -988,15 +1019,15 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
                 x4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
             if (sync()) goto done;
-            double rrl = 0.0;
+            double rrl = 0.0, rpl = 0.0;
             FFAcc rzk{0.f, 0.f};
-            true_residual_ghost<kThreads>(a, P, s0, s1, rrl, rzk, nullptr, false);
+            true_residual_ghost<kThreads>(a, P, s0, s1, rrl, rzk, nullptr, &rpl, false);
             const FF t = rzk.result();
-            double v[2] = {rrl, (double)t.hi + (double)t.lo};
-            group_publish<2>(v, red, part2, rank);
+            double v[3] = {rrl, (double)t.hi + (double)t.lo, rpl};
+            group_publish<3>(v, red, part2, rank);
             if (sync()) goto done;
-            double tt[2];
-            group_reduce0<2>(part2, G, tt);
+            double tt[3];
+            group_reduce0<3>(part2, G, tt);
             if (tid == 0) {
                 FF be;
                 s_flag = sc.replaced(tt, a.max_iter, be);
@@ -1081,6 +1112,8 @@ __global__ void __launch_bounds__(kMixThreads, kMixMinBlocks)
     mixed_solve_ghost<kMixThreads>(a, g, gh, smem);
 }
 
+#include "mixed_slice.cuh"
+
 // Workspace of the ghost plan for layout A on this device: local columns,
 // ghost lists of up to one block per SM, counts, the failure flag.
 size_t ghost_plan_bytes(const nbg_bsr_t& A) {
@@ -1089,7 +1122,7 @@ size_t ghost_plan_bytes(const nbg_bsr_t& A) {
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return 0;
     const size_t G = (size_t)nsm * kMixMinBlocks;
-    return align256(2 * (size_t)A.n_entries) + align256(G * kGhostMax * 4) + align256(G * 4) + 256;
+    return align256(2 * (size_t)A.n_entries) + align256(G * kGhostMax * 4) + align256(G * 8) + 256;
 }
 
 }  // namespace
@@ -1129,22 +1162,20 @@ extern "C" size_t nbg_cg_mixed_layout_workspace_bytes(const nbg_bsr_t* A) {
 }
 
 namespace {
-// The ghost plan for a G-block partition of A, and the launch data of the
-// ghost form when its vectors fit in shared memory at one block per SM:
-// returns 1 and fills gh and *dyn, or 0 (the caller keeps the global-gather
-// form).  plan: the workspace region of ghost_plan_bytes(A).
-int ghost_setup(const nbg_bsr_t& A, unsigned G, char* plan, cudaStream_t s, GhostArgs* gh,
-                size_t* dyn) {
+// The ghost plan for a G-block partition of A and the sizes that its launch
+// needs: returns 1 and fills gh and *widest (entries of the longest slice
+// row), or 0 (the caller keeps a global-gather form).  plan: the
+// workspace region of ghost_plan_bytes(A).
+int ghost_plan(const nbg_bsr_t& A, unsigned G, char* plan, cudaStream_t s, GhostArgs* gh,
+               uint32_t* widest) {
     if (!NBG_MIXED_RESIDENT) return 0;
     uint16_t* lcol = (uint16_t*)plan;
     uint32_t* ids = (uint32_t*)(plan + align256(2 * (size_t)A.n_entries));
     uint32_t* count = ids + (size_t)G * kGhostMax;
-    int* fail = (int*)((char*)count + align256((size_t)G * 4));
-    int dev = 0, nsm = 0, optin = 0;
+    int* fail = (int*)((char*)count + align256((size_t)G * 8));
+    int dev = 0, nsm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
-            cudaSuccess)
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return 0;
     if (G > (unsigned)nsm * kMixMinBlocks) return 0;  // beyond the plan's space
     if (cudaFuncSetAttribute((const void*)k_ghost_plan,
@@ -1154,44 +1185,111 @@ int ghost_setup(const nbg_bsr_t& A, unsigned G, char* plan, cudaStream_t s, Ghos
     if (cudaMemsetAsync(fail, 0, sizeof(int), s) != cudaSuccess) return 0;
     k_ghost_plan<<<G, 1024, kGhostKeys * 4, s>>>(A, lcol, ids, count, fail);
     if (cudaGetLastError() != cudaSuccess) return 0;
-    std::vector<uint32_t> cnt(G);
+    std::vector<uint32_t> cnt(2 * (size_t)G);
     int hfail = 1;
-    if (cudaMemcpyAsync(cnt.data(), count, 4 * (size_t)G, cudaMemcpyDeviceToHost, s) !=
+    if (cudaMemcpyAsync(cnt.data(), count, 8 * (size_t)G, cudaMemcpyDeviceToHost, s) !=
             cudaSuccess ||
         cudaMemcpyAsync(&hfail, fail, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess || hfail)
         return 0;
-    uint32_t scap = 0, pcap = 0, gcap = 0;
+    uint32_t scap = 0, pcap = 0, gcap = 0, ecap = 0;
     for (unsigned b = 0; b < G; b++) {
         const uint32_t s0 = (uint32_t)(((uint64_t)A.n_slices * b) / G);
         const uint32_t s1 = (uint32_t)(((uint64_t)A.n_slices * (b + 1)) / G);
         scap = std::max(scap, 32 * (s1 - s0));
         pcap = std::max(pcap, 32 * (s1 - s0) + cnt[b]);
         gcap = std::max(gcap, cnt[b]);
+        ecap = std::max(ecap, cnt[G + b]);
     }
-    const size_t bytes = 16 * (size_t)pcap + 16 * (size_t)scap + 4 * (size_t)gcap +
-                         (NBG_MIXED_SO_SMEM ? 4 * ((size_t)scap / 32 + 1) : 0);
-    cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, (const void*)k_cg_mixed_ghost) != cudaSuccess ||
-        bytes + fa.sharedSizeBytes > (size_t)optin)
-        return 0;
-    if (cudaFuncSetAttribute((const void*)k_cg_mixed_ghost,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
-        cudaSuccess)
-        return 0;
-    int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void*)k_cg_mixed_ghost,
-                                                      kMixThreads, bytes) != cudaSuccess ||
-        (unsigned)occ * (unsigned)nsm < G)
-        return 0;
     gh->lcol = lcol;
     gh->ids = ids;
     gh->count = count;
     gh->scap = scap;
     gh->pcap = pcap;
     gh->gcap = gcap;
+    *widest = ecap;
+    return 1;
+}
+
+// Whether `bytes` of dynamic shared memory let G blocks of `fn` run at once;
+// sets the kernel's limit to them.
+bool fits_smem(const void* fn, int threads, size_t bytes, unsigned G) {
+    int dev = 0, nsm = 0, optin = 0, occ = 0;
+    cudaFuncAttributes fa;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
+            cudaSuccess ||
+        cudaFuncGetAttributes(&fa, fn) != cudaSuccess || bytes + fa.sharedSizeBytes > (size_t)optin)
+        return false;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) ==
+               cudaSuccess &&
+           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, bytes) ==
+               cudaSuccess &&
+           (uint64_t)occ * (unsigned)nsm >= G;
+}
+
+// The ghost-node form for a G-block partition: 1 and its launch data when the
+// vectors fit in shared memory at one block per SM.
+int ghost_setup(const nbg_bsr_t& A, unsigned G, char* plan, cudaStream_t s, GhostArgs* gh,
+                size_t* dyn) {
+    uint32_t widest;
+    if (!ghost_plan(A, G, plan, s, gh, &widest)) return 0;
+    const size_t bytes = 16 * (size_t)gh->pcap + 16 * (size_t)gh->scap + 4 * (size_t)gh->gcap +
+                         (NBG_MIXED_SO_SMEM ? 4 * ((size_t)gh->scap / 32 + 1) : 0);
+    if (!fits_smem((const void*)k_cg_mixed_ghost, kMixThreads, bytes, G)) return 0;
     *dyn = bytes;
     return 1;
+}
+
+// Blocks of the slice form, 0 when the system is too large for it (a block
+// has at most 32 warps and the grid one block per SM).  Four slices per
+// block, one warp per scheduler, while there are SMs: the sums cost about
+// the same over 17 blocks as over 152, the SpMV's FP32 work grows with the
+// warps that share a scheduler.  Microseconds per iteration with 2, 4, 8, 16
+// and 24 slices per block: 4,290 dof 4.5, 4.4, 4.4, 5.5, 8.5; 16,770 dof
+// 4.5, 4.4, 4.9, 5.9, 8.9.
+unsigned slice_grid(uint32_t n_slices, int nsm) {
+    const unsigned most = std::min((unsigned)nsm, kExactMaxBlocks);
+    if (n_slices > most * (kMixThreads / 32)) return 0;
+    return std::min(most, (n_slices + 3) / 4);
+}
+
+template <int kThreads>
+const void* slice_kernel_of(bool ghost) {
+    return ghost ? (const void*)k_cg_mixed_slice<true, kThreads>
+                 : (const void*)k_cg_mixed_slice<false, kThreads>;
+}
+
+// The instance with the most registers for `threads`.
+const void* slice_kernel(bool ghost, int threads) {
+    return threads <= 512 ? slice_kernel_of<512>(ghost)
+         : threads <= 896 ? slice_kernel_of<896>(ghost)
+                          : slice_kernel_of<kMixThreads>(ghost);
+}
+
+// The slice form with ghosts for a G-block partition: as ghost_setup; the
+// matrix takes what shared memory is left, *keep entries of every row.
+int slice_setup(const nbg_bsr_t& A, unsigned G, int threads, char* plan, cudaStream_t s,
+                GhostArgs* gh, uint32_t* keep, size_t* dyn) {
+    uint32_t widest;
+    if (!ghost_plan(A, G, plan, s, gh, &widest)) return 0;
+    const size_t base = 16 * (size_t)gh->pcap + 16 * (size_t)gh->gcap +
+                        4 * (size_t)((gh->gcap + 3) & ~3u);
+    int dev = 0, optin = 0;
+    cudaFuncAttributes fa;
+    const void* fn = slice_kernel(true, threads);
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
+            cudaSuccess ||
+        cudaFuncGetAttributes(&fa, fn) != cudaSuccess)
+        return 0;
+    if (base + fa.sharedSizeBytes > (size_t)optin) return 0;
+    const size_t left = (size_t)optin - fa.sharedSizeBytes - base;
+    const size_t column = slice_entry_bytes(threads) * (size_t)threads;
+    *keep = (uint32_t)std::min<size_t>(widest, left / column);
+    *dyn = base + column * *keep;
+    return fits_smem(fn, threads, *dyn, G) ? 1 : 0;
 }
 }  // namespace
 
@@ -1237,7 +1335,7 @@ extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint
     unsigned G = 1;
     size_t dyn = 0;
     double hr[5] = {0, 0, 0, 0, 0};
-    cudaError_t e = cudaMemsetAsync(tail, 0, 3 * 256, s);
+    cudaError_t e = cudaMemsetAsync(tail, 0, kMixTail, s);
     if (A->perm) {  // solve in the layout's node order
         double* bp = (double*)(base + mixed_core_bytes(A->N));
         double* xp = bp + align256((size_t)A->N * 8) / 8;
@@ -1248,40 +1346,48 @@ extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint
     }
     GhostArgs gh;
     memset(&gh, 0, sizeof(gh));
+    SliceArgs sl{0, tail + 3 * 256};
     bool ghost = false;
-    if (e == cudaSuccess && plan) {
-        // one block per SM, as the resident global-gather form's first choice
-        int dev = 0, nsm = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess &&
-            cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) {
-            const unsigned want = (A->n_slices + kMixThreads / 32 - 1) / (kMixThreads / 32);
-            G = std::max(1u, std::min((unsigned)nsm * kMixMinBlocks, want));
-            ghost = ghost_setup(*A, G, plan, s, &gh, &dyn) == 1;
-        }
+    int dev = 0, nsm = 0, threads = kMixThreads;
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const unsigned slice_g = NBG_MIXED_RESIDENT ? slice_grid(A->n_slices, nsm) : 0;
+    const void* fn = nullptr;
+    if (e == cudaSuccess && slice_g) {
+        G = slice_g;
+        threads = 32 * (int)((A->n_slices + G - 1) / G);
+        ghost = plan && slice_setup(*A, G, threads, plan, s, &gh, &sl.keep, &dyn) == 1;
+        if (!ghost) dyn = 0;
         (void)cudaGetLastError();  // a plan that could not run leaves the global-gather form
+        fn = slice_kernel(ghost, threads);
+    } else if (e == cudaSuccess && plan) {
+        // one block per SM, as the resident global-gather form's first choice
+        const unsigned want = (A->n_slices + kMixThreads / 32 - 1) / (kMixThreads / 32);
+        G = std::max(1u, std::min((unsigned)nsm * kMixMinBlocks, want));
+        ghost = ghost_setup(*A, G, plan, s, &gh, &dyn) == 1;
+        (void)cudaGetLastError();
+        if (ghost) fn = (const void*)k_cg_mixed_ghost;
     }
-    if (e == cudaSuccess && !ghost)
+    if (e == cudaSuccess && !fn) {
         rc = coop_grid_resident((const void*)k_cg_mixed<true>, A->n_slices,
                                 NBG_MIXED_RESIDENT ? kOwnNodeBytes * 32 : 0, &G, &dyn, kMixThreads,
                                 kMixMinBlocks);
-    if (e == cudaSuccess && rc == NBG_OK && !ghost && dyn == 0)
-        rc = coop_grid((const void*)k_cg_mixed<false>, A->n_slices, &G, kMixThreads);
+        if (rc == NBG_OK && dyn == 0)
+            rc = coop_grid((const void*)k_cg_mixed<false>, A->n_slices, &G, kMixThreads);
+        fn = dyn > 0 ? (const void*)k_cg_mixed<true> : (const void*)k_cg_mixed<false>;
+    }
     a.resident = dyn > 0;
-    const void* fn = ghost ? (const void*)k_cg_mixed_ghost
-                           : a.resident ? (const void*)k_cg_mixed<true>
-                                        : (const void*)k_cg_mixed<false>;
     g.s_begin = 0;
     g.s_end = A->n_slices;
     g.g_base = 0;
     g.g_size = G;
     g.pstride = kMaxBlocks;
     if (ghost) a.keep_pm = keep_permille(*A, 30.0);
-    g_mixed_form = ghost ? NBG_MIXED_GHOST : a.resident ? NBG_MIXED_RESIDENT_ROWS
-                                                       : NBG_MIXED_GLOBAL_ROWS;
+    g_mixed_form = ghost ? NBG_MIXED_GHOST : slice_g || a.resident ? NBG_MIXED_RESIDENT_ROWS
+                                                                  : NBG_MIXED_GLOBAL_ROWS;
     if (e == cudaSuccess && rc == NBG_OK) {
-        void* args[] = {&a, &g, &gh};
-        e = cudaLaunchCooperativeKernel(fn, dim3(G), dim3(kMixThreads),
-                                        args, dyn, s);
+        void* args[] = {&a, &g, &gh, &sl};
+        e = cudaLaunchCooperativeKernel(fn, dim3(G), dim3(threads), args, dyn, s);
         if (e == cudaSuccess && A->perm) e = perm_scatter(A->Nn, A->perm, (const double*)a.u, x, s);
     }
     if (e == cudaSuccess && rc == NBG_OK)

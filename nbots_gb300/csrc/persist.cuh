@@ -268,7 +268,9 @@ __device__ __forceinline__ void group_reduce0(const double* part, uint32_t G, do
     }
 }
 
-// (A x) for node row (s, lane) with FP64 values and FMAs.
+// (A x) for node row (s, lane) with FP64 values: FMAs, or (kRounded) nbots'
+// rounded products and left-to-right sums.
+template <bool kRounded = false>
 __device__ __forceinline__ double2 spmv_row_f64(const nbg_bsr_t& A, uint32_t s, uint32_t lane,
                                                 const double2* __restrict__ xv) {
     const double2* __restrict__ bv = reinterpret_cast<const double2*>(A.b64);
@@ -282,10 +284,15 @@ __device__ __forceinline__ double2 spmv_row_f64(const nbg_bsr_t& A, uint32_t s, 
         const size_t e = (size_t)k * 32 + lane;
         const double2 xc = xv[ld_hint(A.bcol + e, pol)];
         const double2 top = ld_hint(bv + 2 * e, pol), bot = ld_hint(bv + 2 * e + 1, pol);
-        y0 = fma(top.x, xc.x, y0);
-        y0 = fma(top.y, xc.y, y0);
-        y1 = fma(bot.x, xc.x, y1);
-        y1 = fma(bot.y, xc.y, y1);
+        if (kRounded) {
+            y0 = add(add(y0, mul(top.x, xc.x)), mul(top.y, xc.y));
+            y1 = add(add(y1, mul(bot.x, xc.x)), mul(bot.y, xc.y));
+        } else {
+            y0 = fma(top.x, xc.x, y0);
+            y0 = fma(top.y, xc.y, y0);
+            y1 = fma(bot.x, xc.x, y1);
+            y1 = fma(bot.y, xc.y, y1);
+        }
     }
     return make_double2(y0, y1);
 }
