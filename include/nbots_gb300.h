@@ -283,6 +283,11 @@ int nbg_spmv_bsr_f32(const nbg_bsr_t *A, const float *x, float *y, void *stream)
  * iterates within rounding of nbots' own.  NBG_CG_RELATIVE selects
  * ||g|| <= tol ||b||.  x holds x0 on entry. */
 size_t nbg_cg_bsr_workspace_bytes(uint32_t N);
+/* With this much (more: a 16-bit local column per layout entry and per-block
+ * ghost lists) systems of up to 32 slices per SM take the slice form, which
+ * keeps its vectors in registers and its rows' and ghosts' p in shared memory;
+ * ws NULL allocates this size. */
+size_t nbg_cg_bsr_layout_workspace_bytes(const nbg_bsr_t *A);
 int nbg_cg_bsr_f64(const nbg_bsr_t *A, const double *b, double *x, uint32_t max_iter,
                    double tol, unsigned flags, nbg_cg_result_t *result, void *ws,
                    size_t ws_bytes, void *stream);

@@ -119,6 +119,7 @@ SIGS = {
     "nbg_spmv_bsr_f64": ([C.POINTER(Bsr), vp, vp, vp], i32),
     "nbg_spmv_bsr_f32": ([C.POINTER(Bsr), vp, vp, vp], i32),
     "nbg_cg_bsr_workspace_bytes": ([u32], sz),
+    "nbg_cg_bsr_layout_workspace_bytes": ([C.POINTER(Bsr)], sz),
     "nbg_cg_bsr_f64": ([C.POINTER(Bsr), vp, vp, u32, f64, C.c_uint, C.POINTER(CgResult), vp,
                         sz, vp], i32),
     "nbg_spmv_bsr_mixed": ([C.POINTER(Bsr), vp, vp, vp, vp, vp], i32),

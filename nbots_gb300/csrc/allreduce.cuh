@@ -252,16 +252,55 @@ __device__ __forceinline__ void limbs_of(FF v, float scale, int (&l)[kSumWords])
     }
 }
 
+// E of the window |v| < 2^E for an FP64 sum whose last value was `last`;
+// kNoWindow: none.
+constexpr int kNoWindow = -100000;
+__device__ __forceinline__ int window_f64(double last) {
+    const int ex = (int)((__double2hiint(last) >> 20) & 2047) - 1023;
+    return ex < -300 || ex > 300 ? kNoWindow : ex + kLimbBits;
+}
+
+// Limbs of an FP64 value: its significand shifted to units of 2^(E - 100),
+// rounded there.
+__device__ __forceinline__ void limbs_of(double v, int E, int (&l)[kSumWords]) {
+    const long long bits = __double_as_longlong(v);
+    const int ex = (int)(bits >> 52) & 2047;
+    const bool out = E == kNoWindow || ex == 2047 || ex - 1023 >= E;
+    unsigned long long m = (unsigned long long)bits & ((1ull << 52) - 1) | 1ull << 52;
+    // subnormal values and those that a right shift clears count as zero:
+    // 2^-80 of the last sum at most
+    int sh = ex - 1075 - E + kLimbs * kLimbBits;
+    if (out || ex == 0 || sh < -53) {
+        m = 0;
+        sh = 0;
+    }
+    unsigned long long lo, hi = 0;
+    if (sh < 0) {
+        lo = (m + (1ull << (-sh - 1))) >> -sh;
+    } else {
+        lo = m << sh;
+        hi = sh ? m >> (64 - sh) : 0;
+    }
+    constexpr int kMask = (1 << kLimbBits) - 1;
+    const int s = bits < 0 ? -1 : 1;
+    l[4] = s * (int)(lo & kMask);
+    l[3] = s * (int)(lo >> 20 & kMask);
+    l[2] = s * (int)(lo >> 40 & kMask);
+    l[1] = s * (int)((lo >> 60 | hi << 4) & kMask);
+    l[0] = s * (int)(hi >> 16);
+    l[kLimbs] = out;
+}
+
 // A warp's limbs into sh[warp * 16 + value * kSumWords + limb], before a
 // __syncthreads.
 constexpr int kSumShared = 32 * 16;  // ints of sh
-template <int NV>
-__device__ __forceinline__ void exact_begin(const FF (&v)[NV], const float (&scale)[NV], int* sh) {
+template <int NV, class V, class W>
+__device__ __forceinline__ void exact_begin(const V (&v)[NV], const W (&window)[NV], int* sh) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < NV; k++) {
         int l[kSumWords];
-        limbs_of(v[k], scale[k], l);
+        limbs_of(v[k], window[k], l);
 #pragma unroll
         for (int j = 0; j < kSumWords; j++) {
             const int t = __reduce_add_sync(0xffffffffu, l[j]);
@@ -289,7 +328,7 @@ struct ExactSum {
     // or 2 (give up).  Called by one whole warp.
     template <int NV>
     __device__ __forceinline__ int sum(const int* sh, uint32_t n_warps, uint32_t G, int* status,
-                                       const float (&scale)[NV], long long& x, int& e) {
+                                       const int (&window)[NV], long long& x, int& e) {
         const uint32_t lane = threadIdx.x & 31;
         constexpr uint32_t kW = NV * kSumWords;
         // lanes 0-15 add the even warps' words, lanes 16-31 the odd ones'
@@ -340,10 +379,16 @@ struct ExactSum {
         const bool bad = l[kLimbs] != 0 || (m == kLimbBits && (v < 0 ? -v : v) < (1ll << 50));
         const int up = max(__clzll(v < 0 ? ~v : v) - 3, 0);
         x = v << up;
-        e = window_exponent(NV == 2 && k ? scale[NV - 1] : scale[0]) - 4 * kLimbBits - m - up;
+        e = (NV == 2 && k ? window[NV - 1] : window[0]) - 4 * kLimbBits - m - up;
         return __any_sync(0xffffffffu, bad);
     }
 };
+
+// x 2^e in FP64.
+__device__ __forceinline__ double exact_f64(long long x, int e) {
+    if (x == 0) return 0.0;
+    return __longlong_as_double(__double_as_longlong(__ll2double_rn(x)) + ((long long)e << 52));
+}
 
 // x 2^e as a float-float number (|x| < 2^61; |e| small enough that 2^(e + 62)
 // is a float): the leading 31 bits and the 31 below them, each exact in an

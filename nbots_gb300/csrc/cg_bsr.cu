@@ -31,7 +31,10 @@
 //    converged (status 1), reporting the last true residual, that floor.
 // JAC = false is the unpreconditioned CG (q = g).
 #include <cstdint>
+#include <cstring>
 
+#include "allreduce.cuh"
+#include "ghost_plan.cuh"
 #include "perm.cuh"
 #include "persist.cuh"
 
@@ -53,6 +56,79 @@ struct CgBsrArgs {
     unsigned flags;
 };
 
+// Scalar state of one solve, kept by thread 0 of every block (each derives
+// the same values from the same sums).
+struct CgBsrScalars {
+    double gq, gq_old, gg, bb, target2, report, gg_check, gg0, k_limit;
+    uint32_t k, checks;
+
+    __device__ __forceinline__ void clear() {
+        gq = gq_old = gg = bb = target2 = report = gg_check = gg0 = k_limit = 0.0;
+        k = checks = 0;
+    }
+    // The start's sums {g.q, g.g, b.b}; the return value is s_stop.
+    __device__ __forceinline__ int start(const double (&t)[3], const CgBsrArgs& a) {
+        gq = t[0];
+        gg = report = gg0 = t[1];
+        bb = t[2];
+        target2 = (a.flags & NBG_CG_RELATIVE) ? a.tol * a.tol * bb : a.tol * a.tol;
+        return !(gg > target2) || a.max_iter == 0;
+    }
+    // An iteration's new {g.q, g.g}: sets stop, returns beta.
+    template <bool LAGGED>
+    __device__ __forceinline__ double step(double gq_new, double gg_new, const CgBsrArgs& a,
+                                           int& stop) {
+        gq_old = gq;
+        gq = gq_new;
+        const double beta = gq_new / gq_old;
+        k++;
+        if (LAGGED) {
+            const double lag = gg;  // ||g_{k-1}||^2, as nbots tests it
+            gg = gg_new;
+            report = lag;
+            stop = !(lag > target2) || k >= a.max_iter;
+        } else {
+            gg = report = gg_new;
+            stop = !(gg > target2) ? 2 : (k >= a.max_iter ? 1 : 0);
+            // after a failed check the recurrence gets twice the iterations
+            // its rate so far needs to meet the target again; when it hovers
+            // above it instead, the true residual of that check is the FP64
+            // floor
+            if (stop == 0 && checks > 0 && (double)k > k_limit) {
+                stop = 1;
+                report = gg_check;
+            }
+        }
+        return beta;
+    }
+    // The true residual's {g.q, g.g}: sets stop, returns beta from it.
+    __device__ __forceinline__ double checked(double gq_true, double gg_true, const CgBsrArgs& a,
+                                              int& stop) {
+        checks++;
+        gq = gq_true;
+        gg = report = gg_true;
+        // the recurrence fell below the target again but the true residual
+        // did not follow (not even halved since the last check): it sits at
+        // its FP64 floor above the target
+        const bool stalled = checks > 1 && !(gg < 0.25 * gg_check);
+        gg_check = gg;
+        // iterations to go from this residual to the target at the rate of
+        // the k so far (from gg0 to the target)
+        const double need = (double)k * log(gg / target2) / log(gg0 / target2);
+        k_limit = (double)k + 2.0 * need + 100.0;
+        stop = !(gg > target2) || stalled || k >= a.max_iter || checks >= 64;
+        return gq / gq_old;
+    }
+    __device__ __forceinline__ void report_to(const CgBsrArgs& a) const {
+        a.res[0] = (double)k;
+        const int st = ld_volatile(a.status);
+        a.res[1] = st != 0 ? (double)st : (report > target2 ? 1.0 : 0.0);
+        a.res[2] = report;
+        a.res[3] = bb;
+        a.res[4] = (double)checks;
+    }
+};
+
 template <bool JAC>
 __device__ __forceinline__ double2 precond(double2 g, double2 di) {
     return JAC ? make_double2(g.x * di.x, g.y * di.y) : g;
@@ -63,10 +139,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistMinBlocks) k_cg_bsr_f
     __shared__ double buf[3 * kPersistThreads];
     __shared__ double s_coef;  // alpha, then beta
     __shared__ int s_stop;     // 0 iterate, 1 stop, 2 confirm on the true residual first
-    __shared__ struct {
-        double gq, gq_old, gg, bb, target2, report, gg_check, gg0, k_limit;
-        uint32_t k, checks;
-    } sc;  // scalar state, thread 0 only
+    __shared__ CgBsrScalars sc;  // thread 0 only
     const unsigned G = gridDim.x;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t nw = kPersistThreads / 32;
@@ -88,11 +161,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistMinBlocks) k_cg_bsr_f
     // still need them
     double* const part2 = a.part + 3 * kMaxBlocks;
 
-    if (threadIdx.x == 0) {
-        sc.gq = sc.gq_old = sc.gg = sc.bb = sc.target2 = sc.report = sc.gg_check = 0.0;
-        sc.gg0 = sc.k_limit = 0.0;
-        sc.k = sc.checks = 0;
-    }
+    if (threadIdx.x == 0) sc.clear();
     {   // init: g = A x - b, q = g / Aii, p = -q
         double v[3] = {0.0, 0.0, 0.0};  // gq, gg, bb
         for (uint32_t s = s0 + warp; s < s1; s += nw) {
@@ -118,13 +187,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistMinBlocks) k_cg_bsr_f
     {
         double t[3];
         group_reduce0<3>(part2, G, t);
-        if (threadIdx.x == 0) {
-            sc.gq = t[0];
-            sc.gg = sc.report = sc.gg0 = t[1];
-            sc.bb = t[2];
-            sc.target2 = (a.flags & NBG_CG_RELATIVE) ? a.tol * a.tol * sc.bb : a.tol * a.tol;
-            s_stop = !(sc.gg > sc.target2) || a.max_iter == 0;
-        }
+        if (threadIdx.x == 0) s_stop = sc.start(t, a);
         __syncthreads();
     }
     while (!s_stop) {
@@ -179,29 +242,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistMinBlocks) k_cg_bsr_f
         {
             double t2[2];
             group_reduce0<2>(part1, G, t2);
-            if (threadIdx.x == 0) {
-                sc.gq_old = sc.gq;
-                sc.gq = t2[0];
-                s_coef = t2[0] / sc.gq_old;  // beta
-                sc.k++;
-                if (LAGGED) {
-                    const double lag = sc.gg;  // ||g_{k-1}||^2, as nbots tests it
-                    sc.gg = t2[1];
-                    sc.report = lag;
-                    s_stop = !(lag > sc.target2) || sc.k >= a.max_iter;
-                } else {
-                    sc.gg = sc.report = t2[1];
-                    s_stop = !(sc.gg > sc.target2) ? 2 : (sc.k >= a.max_iter ? 1 : 0);
-                    // after a failed check the recurrence gets twice the
-                    // iterations its rate so far needs to meet the target
-                    // again; when it hovers above it instead, the true
-                    // residual of that check is the FP64 floor
-                    if (s_stop == 0 && sc.checks > 0 && (double)sc.k > sc.k_limit) {
-                        s_stop = 1;
-                        sc.report = sc.gg_check;
-                    }
-                }
-            }
+            if (threadIdx.x == 0) s_coef = sc.step<LAGGED>(t2[0], t2[1], a, s_stop);
             __syncthreads();
         }
         if (!LAGGED && s_stop == 2) {
@@ -229,24 +270,7 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistMinBlocks) k_cg_bsr_f
             if (grid_barrier(a.bar, G, blockIdx.x, a.status)) goto done;
             double t2[2];
             group_reduce0<2>(part2, G, t2);
-            if (threadIdx.x == 0) {
-                sc.checks++;
-                sc.gq = t2[0];
-                sc.gg = sc.report = t2[1];
-                s_coef = t2[0] / sc.gq_old;  // beta from the replaced residual
-                // the recurrence fell below the target again but the true
-                // residual did not follow (not even halved since the last
-                // check): it sits at its FP64 floor above the target
-                const bool stalled = sc.checks > 1 && !(sc.gg < 0.25 * sc.gg_check);
-                sc.gg_check = sc.gg;
-                // iterations to go from this residual to the target at the
-                // rate of the k so far (from gg0 to the target)
-                const double need = (double)sc.k * log(sc.gg / sc.target2) /
-                                    log(sc.gg0 / sc.target2);
-                sc.k_limit = (double)sc.k + 2.0 * need + 100.0;
-                s_stop = !(sc.gg > sc.target2) || stalled || sc.k >= a.max_iter ||
-                         sc.checks >= 64;
-            }
+            if (threadIdx.x == 0) s_coef = sc.checked(t2[0], t2[1], a, s_stop);
             __syncthreads();
         }
         if (s_stop) break;
@@ -262,18 +286,24 @@ __global__ void __launch_bounds__(kPersistThreads, kPersistMinBlocks) k_cg_bsr_f
         if (grid_barrier(a.bar, G, blockIdx.x, a.status)) goto done;
     }
 done:
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        a.res[0] = (double)sc.k;
-        int st = ld_volatile(a.status);
-        a.res[1] = st != 0 ? (double)st : (sc.report > sc.target2 ? 1.0 : 0.0);
-        a.res[2] = sc.report;
-        a.res[3] = sc.bb;
-        a.res[4] = (double)sc.checks;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) sc.report_to(a);
 }
 
+struct TrueType {
+    static constexpr bool value = true;
+};
+struct FalseType {
+    static constexpr bool value = false;
+};
+
+#include "cg_bsr_slice.cuh"
+
+// Vectors, partial sums, then what a launch needs at zero: barrier, status
+// and result words and the records and words of the slice form's sums.
+constexpr size_t kBsrTail = 3 * 256 + kArBytes + 2 * kExactBytes;
+
 size_t cg_bsr_core_bytes(uint32_t N) {
-    return 4 * align256((size_t)N * 8) + align256(kMaxBlocks * 3 * 8) * 2 + 3 * 256;
+    return 4 * align256((size_t)N * 8) + align256(kMaxBlocks * 3 * 8) * 2 + kBsrTail;
 }
 
 // plus the permuted copies of b and x for a layout with a node order
@@ -283,6 +313,10 @@ size_t cg_bsr_bytes(uint32_t N) { return cg_bsr_core_bytes(N) + perm_tail_bytes(
 
 extern "C" size_t nbg_cg_bsr_workspace_bytes(uint32_t N) { return cg_bsr_bytes(N); }
 
+extern "C" size_t nbg_cg_bsr_layout_workspace_bytes(const nbg_bsr_t* A) {
+    return A ? cg_bsr_bytes(A->N) + ghost_plan_bytes(*A) : 0;
+}
+
 extern "C" int nbg_cg_bsr_f64(const nbg_bsr_t* A, const double* b, double* x, uint32_t max_iter,
                               double tol, unsigned flags, nbg_cg_result_t* result, void* ws,
                               size_t ws_bytes, void* stream) {
@@ -291,15 +325,18 @@ extern "C" int nbg_cg_bsr_f64(const nbg_bsr_t* A, const double* b, double* x, ui
     if (A->Nn == 0) return NBG_OK;
     if (!A->b64 || ((flags & NBG_CG_JACOBI) && !A->dinv64)) return NBG_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t need = cg_bsr_bytes(A->N);
+    const size_t need = cg_bsr_bytes(A->N), plan_bytes = ghost_plan_bytes(*A);
     void* own = nullptr;
     if (!ws) {
-        NBG_CHECK(cudaMalloc(&own, need));
+        NBG_CHECK(cudaMalloc(&own, need + plan_bytes));
         ws = own;
+        ws_bytes = need + plan_bytes;
     } else if (ws_bytes < need) {
         return NBG_ERR_ARG;
     }
     char* base = (char*)ws;
+    // the slice form when the workspace holds its plan
+    char* const plan = plan_bytes && ws_bytes >= need + plan_bytes ? base + need : nullptr;
     const size_t v = align256((size_t)A->N * 8);
     CgBsrArgs a;
     a.A = *A;
@@ -320,7 +357,7 @@ extern "C" int nbg_cg_bsr_f64(const nbg_bsr_t* A, const double* b, double* x, ui
     int rc = NBG_OK;
     unsigned G = 1;
     double hr[5] = {0, 0, 0, 0, 0};
-    cudaError_t e = cudaMemsetAsync(tail, 0, 3 * 256, s);
+    cudaError_t e = cudaMemsetAsync(tail, 0, kBsrTail, s);
     if (A->perm) {  // solve in the layout's node order
         double* bp = (double*)(base + cg_bsr_core_bytes(A->N));
         double* xp = bp + align256((size_t)A->N * 8) / 8;
@@ -334,10 +371,27 @@ extern "C" int nbg_cg_bsr_f64(const nbg_bsr_t* A, const double* b, double* x, ui
                                    : (const void*)k_cg_bsr_f64<true, false>)
                          : (lagged ? (const void*)k_cg_bsr_f64<false, true>
                                    : (const void*)k_cg_bsr_f64<false, false>);
-    if (e == cudaSuccess) rc = coop_grid(fn, A->n_slices, &G);
+    BsrSliceArgs sl;
+    memset(&sl, 0, sizeof(sl));
+    sl.qrec = (unsigned char*)base;  // over g and q, which the slice form keeps in registers
+    sl.sums = tail + 3 * 256;
+    int threads = kPersistThreads;
+    size_t dyn = 0;
+    bool slice = false;
+    if (e == cudaSuccess && plan) {
+        const void* sfn = nullptr;
+        slice = bsr_slice_setup(*A, jac, lagged, plan, s, &sl, &sfn, &G, &threads, &dyn) == 1;
+        (void)cudaGetLastError();  // a plan that could not run leaves the global form
+        if (slice) fn = sfn;
+    }
+    if (!slice) {
+        threads = kPersistThreads;
+        dyn = 0;
+        if (e == cudaSuccess) rc = coop_grid(fn, A->n_slices, &G);
+    }
     if (e == cudaSuccess && rc == NBG_OK) {
-        void* args[] = {&a};
-        e = cudaLaunchCooperativeKernel(fn, dim3(G), dim3(kPersistThreads), args, 0, s);
+        void* args[] = {&a, &sl};
+        e = cudaLaunchCooperativeKernel(fn, dim3(G), dim3(threads), args, dyn, s);
         if (e == cudaSuccess && A->perm) e = perm_scatter(A->Nn, A->perm, (const double*)a.x, x, s);
     }
     if (e == cudaSuccess && rc == NBG_OK)

@@ -317,7 +317,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (warp == 0) {
                 long long xs;
                 int es;
-                const int st = sum1.sum<1>(s_sum1, nw, G, g.status, scale, xs, es);
+                const int st =
+                    sum1.sum<1>(s_sum1, nw, G, g.status, {window_exponent(scale[0])}, xs, es);
                 if (tid == 0) {
                     s_again = st;
                     if (!st) finish(exact_ff(xs, es));
@@ -366,7 +367,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (warp == 0) {
                 long long xs;
                 int es;
-                const int st = sum2.sum<2>(s_sum2, nw, G, g.status, scale, xs, es);
+                const int st = sum2.sum<2>(
+                    s_sum2, nw, G, g.status,
+                    {window_exponent(scale[0]), window_exponent(scale[1])}, xs, es);
                 const FF t = exact_ff(xs, es);  // r.z in lane 0, |r|^2 in lane 1
                 const FF rrs = {__shfl_sync(0xffffffffu, t.hi, 1), __shfl_sync(0xffffffffu, t.lo, 1)};
                 if (tid == 0) {

@@ -143,7 +143,7 @@ int nbg_fem_damage(nbg_fem_t *f, const nbg_bcs_t *bcs, double E, double nu, doub
 	TRY(nbg_dev_alloc((void **)&w.rws, nbg_residual_workspace_bytes(N) + 8));
 	w.norm2 = w.rws + nbg_residual_workspace_bytes(N) / 8;
 	TRY(nbg_fem_cg_workspace(f));
-	const size_t bws_bytes = nbg_cg_bsr_workspace_bytes(N);
+	const size_t bws_bytes = nbg_cg_bsr_layout_workspace_bytes(&f->bsr);
 	if (blocked)
 		TRY(nbg_dev_alloc((void **)&w.bws, bws_bytes));
 	Eh = malloc(8 * (size_t)(ne ? ne : 1));

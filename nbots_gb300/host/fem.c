@@ -687,7 +687,7 @@ int nbg_fem_solve_fast(nbg_fem_t *f, uint32_t max_iter, double tol, unsigned fla
 {
 	int rc = NBG_OK;
 	TRY(nbg_fem_block_layout(f, NULL));
-	TRY(ensure_ws(f, nbg_cg_bsr_workspace_bytes(f->N)));
+	TRY(ensure_ws(f, nbg_cg_bsr_layout_workspace_bytes(&f->bsr)));
 	TRY(zero_u(f));
 	return nbg_cg_bsr_f64(&f->bsr, f->F, f->u, max_iter, tol, flags, res, f->cg_ws,
 			      f->cg_ws_bytes, f->stream);
@@ -794,7 +794,7 @@ static int solve_rhs(nbg_fem_t *f, const double *b, double *x, double tol, int m
 	if (rc != NBG_OK)
 		return rc;
 	const size_t need = method == NBG_METHOD_MIXED ? nbg_cg_mixed_layout_workspace_bytes(&f->bsr)
-						      : nbg_cg_bsr_workspace_bytes(f->N);
+						      : nbg_cg_bsr_layout_workspace_bytes(&f->bsr);
 	if ((rc = ensure_ws(f, need)) != NBG_OK)
 		return rc;
 	if (method == NBG_METHOD_MIXED) {
