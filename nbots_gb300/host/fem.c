@@ -253,7 +253,7 @@ void nbg_fem_destroy(nbg_fem_t *f)
 	void *p[] = {f->nod, f->K, f->F, f->u, f->strain, f->stress, f->E, f->Ke, f->Fe, f->main_stress,
 		     f->damage,
 		     f->conn, f->row_ptr, f->col_idx, f->inc_ptr, f->inc_elem, f->distorted,
-		     f->inc_local, f->enabled, f->matched, f->status, f->cg_ws,
+		     f->inc_local, f->enabled, f->status, f->cg_ws,
 		     f->slice_off, f->bcol, f->b64, f->dinv64, f->b32, f->dinv32, f->blo, f->bxt,
 		     f->perm, f->iperm, f->simp_rho, f->simp_out, f->simp_e, f->simp_lam};
 	for (size_t i = 0; i < sizeof(p) / sizeof(p[0]); i++)
@@ -295,7 +295,7 @@ int nbg_fem_create_on_csr(nbg_fem_t **out, const nbg_mesh_t *m, uint64_t nnz,
 	TRY(nbg_dev_alloc((void **)&f->strain, 8 * 3 * (ne ? ne : 1) * (nen == 4 ? 4 : 1)));
 	TRY(nbg_dev_alloc((void **)&f->stress, 8 * 3 * (ne ? ne : 1) * (nen == 4 ? 4 : 1)));
 	TRY(nbg_dev_alloc((void **)&f->distorted, 256));
-	TRY(nbg_dev_alloc((void **)&f->matched, 256));
+	f->matched = (unsigned long long *)((char *)f->distorted + 8);  /* read back together */
 	TRY(nbg_dev_alloc((void **)&f->status, 256));
 	TRY(nbg_h2d(f->nod, m->nod, 16 * Nn, stream));
 	TRY(nbg_h2d(f->conn, m->conn, 4 * ne * nen, stream));
@@ -358,7 +358,7 @@ int nbg_fem_create(nbg_fem_t **out, const nbg_mesh_t *m, void *stream)
 	TRY(nbg_dev_alloc((void **)&f->strain, 8 * 3 * ne * (nen == 4 ? 4 : 1)));
 	TRY(nbg_dev_alloc((void **)&f->stress, 8 * 3 * ne * (nen == 4 ? 4 : 1)));
 	TRY(nbg_dev_alloc((void **)&f->distorted, 256));
-	TRY(nbg_dev_alloc((void **)&f->matched, 256));
+	f->matched = (unsigned long long *)((char *)f->distorted + 8);  /* read back together */
 	TRY(nbg_dev_alloc((void **)&f->status, 256));
 	TRY(nbg_dev_alloc((void **)&f->slice_off, 4 * ((size_t)S + 1)));
 	TRY(nbg_dev_alloc(&edg_d, 8 * (size_t)(m->N_edg ? m->N_edg : 1)));
@@ -414,7 +414,7 @@ int nbg_fem_assemble_dev_damage(nbg_fem_t *f, const double *E, double nu, double
 	int rc = NBG_OK;
 	const size_t ne = f->m.N_elem, nen = f->m.nen, nd = 2 * nen;
 	if (!f->Ke) {
-		TRY(nbg_dev_alloc((void **)&f->Ke, 8 * nd * nd * (ne ? ne : 1)));
+		TRY(nbg_dev_alloc((void **)&f->Ke, nbg_fem_element_bytes(nen) * (ne ? ne : 1)));
 		TRY(nbg_dev_alloc((void **)&f->Fe, 8 * nd * (ne ? ne : 1)));
 	}
 	f->nu = nu;
@@ -423,27 +423,22 @@ int nbg_fem_assemble_dev_damage(nbg_fem_t *f, const double *E, double nu, double
 		TRY(nbg_h2d(f->E, E, 8 * ne, f->stream));
 	if (enabled)
 		TRY(nbg_h2d(f->enabled, enabled, ne, f->stream));
-	uint32_t init = 0xffffffffu;
-	unsigned long long zero = 0;
-	TRY(nbg_h2d(f->distorted, &init, 4, f->stream));
-	TRY(nbg_h2d(f->matched, &zero, 8, f->stream));
+	TRY(nbg_memset(f->distorted, 0xff, 4, f->stream));
+	TRY(nbg_memset(f->matched, 0, 8, f->stream));
 	double gx = gravity ? gravity[0] : 0.0, gy = gravity ? gravity[1] : 0.0;
-	TRY(nbg_element_stiffness_damage_f64((uint32_t)nen, (uint32_t)ne, f->nod, f->conn, f->E,
-					     nu, thickness, density, self_weight, gx, gy,
-					     enabled ? f->enabled : NULL, damage, f->Ke, f->Fe,
-					     f->distorted, f->stream));
-	uint32_t dist_h = 0;
-	TRY(nbg_d2h(&dist_h, f->distorted, 4, f->stream));
+	TRY(nbg_fem_element_blocks((uint32_t)nen, (uint32_t)ne, f->nod, f->conn, f->E, nu, thickness,
+				   density, self_weight, gx, gy, enabled ? f->enabled : NULL, damage,
+				   f->Ke, f->Fe, f->distorted, f->stream));
+	/* does nothing after a distorted element */
+	TRY(nbg_fem_gather_blocks((uint32_t)nen, f->m.N_nod, (uint32_t)ne, f->inc_ptr, f->inc_elem,
+				  f->inc_local, f->row_ptr, f->col_idx, f->conn, f->Ke, f->Fe,
+				  self_weight, f->K, f->F, f->matched, f->distorted, f->stream));
+	struct { uint32_t distorted, pad; unsigned long long matched; } st;
+	TRY(nbg_d2h(&st, f->distorted, sizeof(st), f->stream));
 	TRY(nbg_stream_sync(f->stream));
-	if (dist_h != 0xffffffffu)
+	if (st.distorted != 0xffffffffu)
 		return NBG_DISTORTED;
-	TRY(nbg_gather_assemble_f64((uint32_t)nen, f->m.N_nod, (uint32_t)ne, f->inc_ptr,
-				    f->inc_elem, f->inc_local, f->row_ptr, f->col_idx, f->Ke,
-				    f->Fe, f->K, f->F, f->matched, f->stream));
-	unsigned long long matched = 0;
-	TRY(nbg_d2h(&matched, f->matched, 8, f->stream));
-	TRY(nbg_stream_sync(f->stream));
-	if (matched != (unsigned long long)ne * nen * nen)
+	if (st.matched != (unsigned long long)ne * nen * nen)
 		return NBG_ERR_PATTERN;
 	return NBG_OK;
 fail:

@@ -53,6 +53,21 @@ int nbg_fem_create_on_csr(nbg_fem_t **out, const nbg_mesh_t *m, uint64_t nnz,
 int nbg_fem_assemble_dev_damage(nbg_fem_t *f, const double *E, double nu, double thickness,
 				double density, int self_weight, const double gravity[2],
 				const uint8_t *enabled, const double *damage);
+/* Element matrices as node blocks (nbg_fem_element_bytes per element) and
+ * loads (one double per element without self weight, else 2 nen N_elem), and
+ * their gather, which does nothing when *distorted is set (assemble.cu). */
+size_t nbg_fem_element_bytes(uint32_t nen);
+int nbg_fem_element_blocks(uint32_t nen, uint32_t N_elem, const double *nod, const uint32_t *conn,
+			   const double *E, double nu, double thickness, double density,
+			   int self_weight, double gx, double gy, const uint8_t *enabled,
+			   const double *damage, double *Ke, double *Fe, uint32_t *distorted,
+			   void *stream);
+int nbg_fem_gather_blocks(uint32_t nen, uint32_t N_nod, uint32_t N_elem, const uint32_t *inc_ptr,
+			  const uint32_t *inc_elem, const uint8_t *inc_local,
+			  const uint32_t *row_ptr, const uint32_t *col_idx, const uint32_t *conn,
+			  const double *Ke, const double *Fe, int self_weight, double *K, double *F,
+			  unsigned long long *matched, const uint32_t *distorted, void *stream);
+
 /* Grow f's CG workspace to what nbg_cg_f64 needs for f->N dofs. */
 int nbg_fem_cg_workspace(nbg_fem_t *f);
 
