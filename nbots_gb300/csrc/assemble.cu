@@ -533,6 +533,26 @@ __global__ void k_increments(uint32_t n_groups, const uint32_t* __restrict__ idx
     F[idx[g]] = f;
 }
 
+__global__ void k_pick_nodes(uint32_t n, const uint32_t* __restrict__ ids,
+                             const double2* __restrict__ nod, double2* __restrict__ xy) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) xy[k] = nod[ids[k]];
+}
+
+// Offsets of every dof's events in the list sorted by dof (a binary search
+// each: 10 steps for a clamped edge of 500 nodes).
+__global__ void k_event_ptr(uint32_t N, uint32_t n_ev, const uint32_t* __restrict__ ev_dof,
+                            uint32_t* __restrict__ ev_ptr) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > N) return;
+    uint32_t lo = 0, hi = n_ev;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (ev_dof[mid] < i) lo = mid + 1; else hi = mid;
+    }
+    ev_ptr[i] = lo;
+}
+
 constexpr int kMaxRowEvents = 96;
 
 // Thread per row j: replay, in global event order, every Dirichlet event
@@ -737,6 +757,23 @@ extern "C" int nbg_fem_element_blocks(uint32_t nen, uint32_t N_elem, const doubl
     if (N_elem == 0) return NBG_OK;
     return launch_elements<true>(nen, N_elem, nod, conn, E, nu, thickness, density, self_weight, gx,
                                  gy, enabled, damage, Ke, Fe, distorted, (cudaStream_t)stream);
+}
+
+extern "C" int nbg_fem_pick_nodes(uint32_t n, const uint32_t* ids, const double* nod, double* xy,
+                                  void* stream) {
+    if (n == 0) return NBG_OK;
+    k_pick_nodes<<<nblk(n, 256), 256, 0, (cudaStream_t)stream>>>(
+        n, ids, reinterpret_cast<const double2*>(nod), reinterpret_cast<double2*>(xy));
+    NBG_CHECK(cudaGetLastError());
+    return NBG_OK;
+}
+
+extern "C" int nbg_fem_event_ptr(uint32_t N, uint32_t n_ev, const uint32_t* ev_dof,
+                                 uint32_t* ev_ptr, void* stream) {
+    k_event_ptr<<<nblk((uint64_t)N + 1, 256), 256, 0, (cudaStream_t)stream>>>(N, n_ev, ev_dof,
+                                                                             ev_ptr);
+    NBG_CHECK(cudaGetLastError());
+    return NBG_OK;
 }
 
 extern "C" int nbg_fem_gather_blocks(uint32_t nen, uint32_t N_nod, uint32_t N_elem,

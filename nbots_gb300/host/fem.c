@@ -254,7 +254,7 @@ void nbg_fem_destroy(nbg_fem_t *f)
 		     f->damage,
 		     f->conn, f->row_ptr, f->col_idx, f->inc_ptr, f->inc_elem, f->distorted,
 		     f->inc_local, f->enabled, f->status, f->cg_ws,
-		     f->slice_off, f->bcol, f->b64, f->dinv64, f->b32, f->dinv32, f->blo, f->bxt,
+		     f->bc_buf, f->ev_ptr, f->slice_off, f->bcol, f->b64, f->dinv64, f->b32, f->dinv32, f->blo, f->bxt,
 		     f->perm, f->iperm, f->simp_rho, f->simp_out, f->simp_e, f->simp_lam};
 	for (size_t i = 0; i < sizeof(p) / sizeof(p[0]); i++)
 		nbg_dev_free(p[i]);
@@ -445,98 +445,162 @@ fail:
 	return rc;
 }
 
+/* (index, position) pairs in ascending order, positions within an index in
+ * ascending order: one key each. */
+static int cmp_u64(const void *a, const void *b)
+{
+	const uint64_t x = *(const uint64_t *)a, y = *(const uint64_t *)b;
+	return x < y ? -1 : (x > y);
+}
+
+static int sorted_keys(uint32_t n, const uint32_t *idx, uint32_t N, uint64_t **out)
+{
+	uint64_t *k = malloc(sizeof(uint64_t) * (size_t)(n ? n : 1));
+	if (!k)
+		return NBG_ERR_NOMEM;
+	int sorted = 1;
+	for (uint32_t i = 0; i < n; i++) {
+		if (idx[i] >= N) {
+			free(k);
+			return NBG_ERR_ARG;
+		}
+		k[i] = (uint64_t)idx[i] << 32 | i;
+		sorted &= i == 0 || k[i - 1] < k[i];
+	}
+	if (!sorted)
+		qsort(k, n, sizeof(uint64_t), cmp_u64);
+	*out = k;
+	return NBG_OK;
+}
+
+/* The node coordinates that the plan reads (segment lengths of Neumann
+ * conditions), in an array indexed by node: all of them, or, when fewer than
+ * a quarter are read, only those (the pages of the others are never
+ * touched).  At 1M dof and one loaded edge the whole download and its fresh
+ * pages took 1 ms. */
+static int plan_coordinates(nbg_fem_t *f, const nbg_bcs_t *b, double **out)
+{
+	int rc = NBG_OK;
+	const size_t Nn = f->m.N_nod;
+	size_t n = 0;
+	void *dev = NULL;
+	uint32_t *ids = NULL;
+	double *got = NULL, *nod = NULL;
+	for (uint32_t a = 0; a < b->N_bc; a++)
+		if (b->bc[a].kind == 1 && b->bc[a].where == 1 && b->bc[a].id < b->N_sgm)
+			n += b->sgm_ptr[b->bc[a].id + 1] - b->sgm_ptr[b->bc[a].id];
+	nod = malloc(16 * Nn);
+	if (!nod)
+		return NBG_ERR_NOMEM;
+	if (4 * n >= Nn) {
+		TRY(nbg_d2h(nod, f->nod, 16 * Nn, f->stream));
+		TRY(nbg_stream_sync(f->stream));
+	} else if (n) {
+		ids = malloc(4 * n);
+		got = malloc(16 * n);
+		if (!ids || !got)
+			TRY(NBG_ERR_NOMEM);
+		size_t k = 0;
+		for (uint32_t a = 0; a < b->N_bc; a++) {
+			const nbg_bc_t *c = &b->bc[a];
+			if (c->kind != 1 || c->where != 1 || c->id >= b->N_sgm)
+				continue;
+			for (uint32_t i = b->sgm_ptr[c->id]; i < b->sgm_ptr[c->id + 1]; i++) {
+				if (b->sgm_nodes[i] >= Nn)
+					TRY(NBG_ERR_ARG);
+				ids[k++] = b->sgm_nodes[i];
+			}
+		}
+		TRY(nbg_dev_alloc(&dev, 20 * n + 16));
+		double *xy = dev;
+		uint32_t *dids = (uint32_t *)(xy + 2 * n);
+		TRY(nbg_h2d(dids, ids, 4 * n, f->stream));
+		TRY(nbg_fem_pick_nodes((uint32_t)n, dids, f->nod, xy, f->stream));
+		TRY(nbg_d2h(got, xy, 16 * n, f->stream));
+		TRY(nbg_stream_sync(f->stream));
+		for (size_t i = 0; i < n; i++) {
+			nod[2 * (size_t)ids[i]] = got[2 * i];
+			nod[2 * (size_t)ids[i] + 1] = got[2 * i + 1];
+		}
+	}
+	*out = nod;
+	nod = NULL;
+fail:
+	nbg_dev_free(dev);
+	free(ids);
+	free(got);
+	free(nod);
+	return rc;
+}
+
 int nbg_fem_apply_bcs(nbg_fem_t *f, const nbg_bcs_t *b, double factor)
 {
 	int rc = NBG_OK;
 	plan_t p;
 	memset(&p, 0, sizeof(p));  /* the fail path frees its arrays */
-	uint32_t *gidx = NULL, *gptr = NULL, *order = NULL, *cnt = NULL;
-	uint32_t *ev_ptr = NULL, *ev_of = NULL;
-	double *ginc = NULL;
-	void *d_gidx = NULL, *d_gptr = NULL, *d_ginc = NULL, *d_evptr = NULL, *d_evof = NULL,
-	     *d_evval = NULL;
+	uint64_t *ki = NULL, *ke = NULL;
+	char *h = NULL;
 	nbg_mesh_t mh = f->m;
-	/* segment lengths need the coordinates on the host */
-	double *nod = malloc(16 * (size_t)f->m.N_nod);
-	if (!nod)
-		return NBG_ERR_NOMEM;
-	TRY(nbg_d2h(nod, f->nod, 16 * (size_t)f->m.N_nod, f->stream));
-	TRY(nbg_stream_sync(f->stream));
+	double *nod = NULL;
+	const uint32_t N = f->N;
+	TRY(plan_coordinates(f, b, &nod));
 	mh.nod = nod;
 	TRY(build_plan(&mh, b, factor, &p));
-
-	const uint32_t N = f->N;
-	if (p.n_inc) {
-		/* group increments by index, keeping their order within a group */
-		cnt = calloc((size_t)N + 1, sizeof(uint32_t));
-		order = malloc(p.n_inc * sizeof(uint32_t));
-		ginc = malloc(p.n_inc * sizeof(double));
-		if (!cnt || !order || !ginc)
-			TRY(NBG_ERR_NOMEM);
-		for (uint32_t k = 0; k < p.n_inc; k++) {
-			if (p.inc_idx[k] >= N)
-				TRY(NBG_ERR_ARG);
-			cnt[p.inc_idx[k] + 1]++;
+	/* increments grouped by index, keeping their order within a group, and
+	 * events by dof: sorted lists, no array over all dofs.  One buffer:
+	 * increments, event values, group indices, group offsets, event dofs,
+	 * event numbers */
+	TRY(sorted_keys(p.n_inc, p.inc_idx, N, &ki));
+	TRY(sorted_keys(p.n_ev, p.ev_dof, N, &ke));
+	uint32_t ng = 0;
+	for (uint32_t k = 0; k < p.n_inc; k++)
+		ng += k == 0 || ki[k] >> 32 != ki[k - 1] >> 32;
+	const size_t o_val = 8 * (size_t)p.n_inc, o_idx = o_val + 8 * (size_t)p.n_ev,
+		     o_ptr = o_idx + 4 * (size_t)ng, o_dof = o_ptr + 4 * ((size_t)ng + 1),
+		     o_of = o_dof + 4 * (size_t)p.n_ev, bytes = o_of + 4 * (size_t)p.n_ev;
+	h = malloc(bytes);
+	if (!h)
+		TRY(NBG_ERR_NOMEM);
+	double *ginc = (double *)h;
+	uint32_t *gidx = (uint32_t *)(h + o_idx), *gptr = (uint32_t *)(h + o_ptr);
+	uint32_t *dof = (uint32_t *)(h + o_dof), *of = (uint32_t *)(h + o_of);
+	uint32_t g = 0;
+	for (uint32_t k = 0; k < p.n_inc; k++) {
+		ginc[k] = p.inc_val[(uint32_t)ki[k]];
+		if (k == 0 || ki[k] >> 32 != ki[k - 1] >> 32) {
+			gidx[g] = (uint32_t)(ki[k] >> 32);
+			gptr[g++] = k;
 		}
-		uint32_t ng = 0;
-		for (uint32_t i = 0; i < N; i++)
-			ng += cnt[i + 1] != 0;
-		gidx = malloc(ng * sizeof(uint32_t));
-		gptr = malloc((ng + 1) * sizeof(uint32_t));
-		if (!gidx || !gptr)
-			TRY(NBG_ERR_NOMEM);
-		for (uint32_t i = 0; i < N; i++)
-			cnt[i + 1] += cnt[i];
-		for (uint32_t k = 0; k < p.n_inc; k++)
-			ginc[cnt[p.inc_idx[k]]++] = p.inc_val[k];
-		/* cnt[i] is now the end of index i's run */
-		uint32_t g = 0, start = 0;
-		gptr[0] = 0;
-		for (uint32_t i = 0; i < N; i++) {
-			if (cnt[i] != start) {
-				gidx[g] = i;
-				gptr[g + 1] = cnt[i];
-				g++;
-				start = cnt[i];
-			}
-		}
-		TRY(nbg_dev_alloc(&d_gidx, 4 * (size_t)ng));
-		TRY(nbg_dev_alloc(&d_gptr, 4 * ((size_t)ng + 1)));
-		TRY(nbg_dev_alloc(&d_ginc, 8 * (size_t)p.n_inc));
-		TRY(nbg_h2d(d_gidx, gidx, 4 * (size_t)ng, f->stream));
-		TRY(nbg_h2d(d_gptr, gptr, 4 * ((size_t)ng + 1), f->stream));
-		TRY(nbg_h2d(d_ginc, ginc, 8 * (size_t)p.n_inc, f->stream));
-		TRY(nbg_apply_increments_f64(ng, d_gidx, d_gptr, d_ginc, f->F, f->stream));
 	}
+	gptr[ng] = p.n_inc;
+	if (p.n_ev)
+		memcpy(h + o_val, p.ev_val, 8 * (size_t)p.n_ev);
+	for (uint32_t k = 0; k < p.n_ev; k++) {
+		dof[k] = (uint32_t)(ke[k] >> 32);
+		of[k] = (uint32_t)ke[k];
+	}
+	/* kept across calls */
+	if (f->bc_bytes < bytes) {
+		nbg_dev_free(f->bc_buf);
+		f->bc_buf = NULL;
+		f->bc_bytes = 0;
+		TRY(nbg_dev_alloc(&f->bc_buf, bytes));
+		f->bc_bytes = bytes;
+	}
+	if (p.n_ev && !f->ev_ptr)
+		TRY(nbg_dev_alloc((void **)&f->ev_ptr, 4 * ((size_t)N + 1)));
+	char *d = f->bc_buf;
+	if (p.n_inc || p.n_ev)
+		TRY(nbg_h2d(d, h, bytes, f->stream));
+	if (p.n_inc)
+		TRY(nbg_apply_increments_f64(ng, (uint32_t *)(d + o_idx), (uint32_t *)(d + o_ptr),
+					     (double *)d, f->F, f->stream));
 	if (p.n_ev) {
-		ev_ptr = calloc((size_t)N + 1, sizeof(uint32_t));
-		ev_of = malloc(p.n_ev * sizeof(uint32_t));
-		if (!ev_ptr || !ev_of)
-			TRY(NBG_ERR_NOMEM);
-		for (uint32_t k = 0; k < p.n_ev; k++) {
-			if (p.ev_dof[k] >= N)
-				TRY(NBG_ERR_ARG);
-			ev_ptr[p.ev_dof[k] + 1]++;
-		}
-		for (uint32_t i = 0; i < N; i++)
-			ev_ptr[i + 1] += ev_ptr[i];
-		uint32_t *pos = malloc(((size_t)N + 1) * sizeof(uint32_t));
-		if (!pos)
-			TRY(NBG_ERR_NOMEM);
-		memcpy(pos, ev_ptr, ((size_t)N + 1) * sizeof(uint32_t));
-		for (uint32_t k = 0; k < p.n_ev; k++)
-			ev_of[pos[p.ev_dof[k]]++] = k;
-		free(pos);
-		int zero = 0;
-		TRY(nbg_h2d(f->status, &zero, sizeof(int), f->stream));
-		TRY(nbg_dev_alloc(&d_evptr, 4 * ((size_t)N + 1)));
-		TRY(nbg_dev_alloc(&d_evof, 4 * (size_t)p.n_ev));
-		TRY(nbg_dev_alloc(&d_evval, 8 * (size_t)p.n_ev));
-		TRY(nbg_h2d(d_evptr, ev_ptr, 4 * ((size_t)N + 1), f->stream));
-		TRY(nbg_h2d(d_evof, ev_of, 4 * (size_t)p.n_ev, f->stream));
-		TRY(nbg_h2d(d_evval, p.ev_val, 8 * (size_t)p.n_ev, f->stream));
-		TRY(nbg_dirichlet_f64(N, f->row_ptr, f->col_idx, f->K, f->F, d_evptr, d_evof,
-				      d_evval, f->status, f->stream));
+		TRY(nbg_memset(f->status, 0, sizeof(int), f->stream));
+		TRY(nbg_fem_event_ptr(N, p.n_ev, (uint32_t *)(d + o_dof), f->ev_ptr, f->stream));
+		TRY(nbg_dirichlet_f64(N, f->row_ptr, f->col_idx, f->K, f->F, f->ev_ptr,
+				      (uint32_t *)(d + o_of), (double *)(d + o_val), f->status,
+				      f->stream));
 		int st = 0;
 		TRY(nbg_d2h(&st, f->status, sizeof(int), f->stream));
 		TRY(nbg_stream_sync(f->stream));
@@ -545,11 +609,14 @@ int nbg_fem_apply_bcs(nbg_fem_t *f, const nbg_bcs_t *b, double factor)
 	}
 	TRY(nbg_stream_sync(f->stream));
 fail:
+	/* the copy from h may still be under way when a later call failed */
+	if (rc != NBG_OK && h)
+		nbg_stream_sync(f->stream);
 	plan_free(&p);
-	free(nod); free(cnt); free(order); free(ginc); free(gidx); free(gptr);
-	free(ev_ptr); free(ev_of);
-	nbg_dev_free(d_gidx); nbg_dev_free(d_gptr); nbg_dev_free(d_ginc);
-	nbg_dev_free(d_evptr); nbg_dev_free(d_evof); nbg_dev_free(d_evval);
+	free(ki);
+	free(ke);
+	free(h);
+	free(nod);
 	return rc;
 }
 
@@ -574,13 +641,7 @@ int nbg_fem_solve(nbg_fem_t *f, uint32_t max_iter, double tol, unsigned flags,
 	int rc = nbg_fem_cg_workspace(f);
 	if (rc != NBG_OK)
 		return rc;
-	double *zero = calloc(f->N ? f->N : 1, sizeof(double));
-	if (!zero)
-		return NBG_ERR_NOMEM;
-	rc = nbg_h2d(f->u, zero, 8 * (size_t)f->N, f->stream);
-	if (rc == NBG_OK)
-		rc = nbg_stream_sync(f->stream);
-	free(zero);
+	rc = nbg_memset(f->u, 0, 8 * (size_t)f->N, f->stream);
 	if (rc != NBG_OK)
 		return rc;
 	return nbg_cg_f64(f->N, f->row_ptr, f->col_idx, f->K, f->F, f->u, max_iter, tol, flags,
@@ -621,7 +682,8 @@ fail:
 	return rc;
 }
 
-int nbg_fem_block_layout(nbg_fem_t *f, nbg_bsr_t *out)
+/* The layout refilled on the stream. */
+static int fill_layout(nbg_fem_t *f)
 {
 	int rc = NBG_OK;
 	if (!f->bsr_ok)
@@ -644,24 +706,24 @@ int nbg_fem_block_layout(nbg_fem_t *f, nbg_bsr_t *out)
 		f->bsr.dinv32 = f->dinv32;
 	}
 	TRY(nbg_bsr_fill(&f->bsr, f->row_ptr, f->col_idx, f->K, f->stream));
-	TRY(nbg_stream_sync(f->stream));
-	if (out)
-		*out = f->bsr;
 	return NBG_OK;
 fail:
 	return rc;
 }
 
-static int zero_u(nbg_fem_t *f)
+int nbg_fem_block_layout(nbg_fem_t *f, nbg_bsr_t *out)
 {
-	double *zero = calloc(f->N ? f->N : 1, sizeof(double));
-	if (!zero)
-		return NBG_ERR_NOMEM;
-	int rc = nbg_h2d(f->u, zero, 8 * (size_t)f->N, f->stream);
+	int rc = fill_layout(f);
 	if (rc == NBG_OK)
 		rc = nbg_stream_sync(f->stream);
-	free(zero);
+	if (rc == NBG_OK && out)
+		*out = f->bsr;
 	return rc;
+}
+
+static int zero_u(nbg_fem_t *f)
+{
+	return nbg_memset(f->u, 0, 8 * (size_t)f->N, f->stream);
 }
 
 static int ensure_ws(nbg_fem_t *f, size_t need)
@@ -681,7 +743,7 @@ int nbg_fem_solve_fast(nbg_fem_t *f, uint32_t max_iter, double tol, unsigned fla
 		       nbg_cg_result_t *res)
 {
 	int rc = NBG_OK;
-	TRY(nbg_fem_block_layout(f, NULL));
+	TRY(fill_layout(f));
 	TRY(ensure_ws(f, nbg_cg_bsr_layout_workspace_bytes(&f->bsr)));
 	TRY(zero_u(f));
 	return nbg_cg_bsr_f64(&f->bsr, f->F, f->u, max_iter, tol, flags, res, f->cg_ws,
@@ -694,7 +756,7 @@ int nbg_fem_solve_mixed(nbg_fem_t *f, uint32_t max_iter, double tol, double delt
 			unsigned flags, nbg_mixed_result_t *res)
 {
 	int rc = NBG_OK;
-	TRY(nbg_fem_block_layout(f, NULL));
+	TRY(fill_layout(f));
 	TRY(ensure_ws(f, nbg_cg_mixed_layout_workspace_bytes(&f->bsr)));
 	TRY(zero_u(f));
 	return nbg_cg_mixed(&f->bsr, f->F, f->u, max_iter, tol, delta, flags, res, f->cg_ws,
@@ -785,7 +847,7 @@ int nbg_fem_upload(nbg_fem_t *f, int what, const void *host)
 static int solve_rhs(nbg_fem_t *f, const double *b, double *x, double tol, int method,
 		     uint32_t *iters)
 {
-	int rc = nbg_fem_block_layout(f, NULL);
+	int rc = fill_layout(f);
 	if (rc != NBG_OK)
 		return rc;
 	const size_t need = method == NBG_METHOD_MIXED ? nbg_cg_mixed_layout_workspace_bytes(&f->bsr)

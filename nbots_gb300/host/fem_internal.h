@@ -34,6 +34,9 @@ struct nbg_fem {
 	int block_order;           /* NBG_ORDER_* */
 	uint32_t block_sigma;      /* SELL-C-sigma window, 0: default */
 	uint32_t *perm, *iperm;    /* the block layout's node order, or NULL */
+	void *bc_buf;              /* boundary-condition lists on the device, kept */
+	size_t bc_bytes;
+	uint32_t *ev_ptr;          /* per dof: its first event, N + 1 */
 	double *simp_rho, *simp_out, *simp_e, *simp_lam;  /* nbg_fem_simp buffers */
 	int borrowed_csr;          /* row_ptr, col_idx and K belong to the caller */
 };
@@ -67,6 +70,13 @@ int nbg_fem_gather_blocks(uint32_t nen, uint32_t N_nod, uint32_t N_elem, const u
 			  const uint32_t *row_ptr, const uint32_t *col_idx, const uint32_t *conn,
 			  const double *Ke, const double *Fe, int self_weight, double *K, double *F,
 			  unsigned long long *matched, const uint32_t *distorted, void *stream);
+
+/* xy[2 k] = nod of node ids[k]; ev_ptr[i] = how many of the ascending
+ * ev_dof[n_ev] are below i, i = 0 .. N (device arrays, assemble.cu). */
+int nbg_fem_pick_nodes(uint32_t n, const uint32_t *ids, const double *nod, double *xy,
+		       void *stream);
+int nbg_fem_event_ptr(uint32_t N, uint32_t n_ev, const uint32_t *ev_dof, uint32_t *ev_ptr,
+		      void *stream);
 
 /* Grow f's CG workspace to what nbg_cg_f64 needs for f->N dofs. */
 int nbg_fem_cg_workspace(nbg_fem_t *f);
