@@ -12,6 +12,9 @@
 
 #include "nbots_gb300.h"
 
+/* csrc/spmv.cu: n doubles of coherent host memory to the device, by a kernel */
+int nbg_copy_in_f64(size_t n, const double *src, double *dst, void *stream);
+
 struct nbg_solver {
 	void *stream;
 	int host_direct;  /* kernels write the caller's host memory directly */
@@ -201,9 +204,13 @@ int nbg_solver_multiply(nbg_solver_t *s, const double *in, double *out)
 	 * NVLink-C2C), the kernel writes the product there itself, overlapping
 	 * the transfer with the FP64-bound SpMV (1M dof: 0.18 against 0.22 ms
 	 * with a copy back; reading x there too was slower, 0.27 ms, so x is
-	 * copied in) */
+	 * copied in).  A kernel copies it from 128 KiB on: at the same rate as
+	 * cudaMemcpyAsync, but the host does not wait for it before it launches
+	 * the product (1M dof 0.152 -> 0.138 ms, 66,306 dof 35 -> 28 us; 4,290
+	 * dof 20.7 against 23.5 us) */
 	const int direct = s->host_direct;
-	int rc = nbg_h2d(s->x, in, 8 * (size_t)s->N, s->stream);
+	int rc = direct && s->N >= 16384 ? nbg_copy_in_f64(s->N, in, s->x, s->stream)
+			: nbg_h2d(s->x, in, 8 * (size_t)s->N, s->stream);
 	if (rc == NBG_OK)
 		rc = nbg_spmv_csr_f64(s->N, s->rp, s->ci, s->val, s->x, direct ? out : s->b,
 				      s->stream);
