@@ -324,9 +324,10 @@ struct ExactSum {
     // The block's limbs are in sh; the sums of NV (1 or 2) values over the
     // grid's G <= 255 blocks, value 0 in the even lanes and value 1 in the odd
     // ones (one value: in every lane), as an integer x of 61 bits and an
-    // exponent e: x 2^e.  Returns 0, 1 (outside the window: sum again by records)
+    // exponent e: x 2^e.  kFence: the sum is also a barrier for the block's
+    // plain loads and stores (release before it, acquire after it).  Returns 0, 1 (outside the window: sum again by records)
     // or 2 (give up).  Called by one whole warp.
-    template <int NV>
+    template <int NV, bool kFence = false>
     __device__ __forceinline__ int sum(const int* sh, uint32_t n_warps, uint32_t G, int* status,
                                        const int (&window)[NV], long long& x, int& e) {
         const uint32_t lane = threadIdx.x & 31;
@@ -342,6 +343,7 @@ struct ExactSum {
         unsigned long long* const p = words + 16 * h + lane;
         unsigned long long d = 0;
         const unsigned long long before = lane < kW ? last[h][lane] : 0;
+        if (kFence) __threadfence();
         if (lane < kW) {
             const unsigned long long add = (1ull << 56) + (unsigned long long)(mine + (1ll << 32));
             asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(add) : "memory");
@@ -356,6 +358,7 @@ struct ExactSum {
             if (__all_sync(0xffffffffu, ok)) break;
             if (__any_sync(0xffffffffu, lim.expired(status))) return 2;
         }
+        if (kFence) __threadfence();
         const long long t = (long long)((d - before) & ((1ull << 56) - 1)) - ((long long)G << 32);
         if (lane < kW) last[h][lane] = d;
         if (lane == 0) half = h ^ 1;

@@ -37,6 +37,7 @@
 #include <cstdint>
 #include <cstring>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "allreduce.cuh"
@@ -90,9 +91,10 @@ constexpr int kUnroll = NBG_MIXED_UNROLL;
 #endif
 #ifndef NBG_L2_KEEP
 // percent of L2 for the matrix part kept between iterations (1M-dof ghost
-// form: 0.2500 s at 40, 0.2560 at 50, 0.2644 at 60, 0.251-0.253 at 10-30:
-// the rest of L2 holds the vectors)
-#define NBG_L2_KEEP 40
+// form, us per iteration: 32.7 at 40, 31.3 at 35, 31.2 at 30, 32.7 at 25, 34.0
+// at 20: the rest of L2 holds the vectors); none for streams of over twice the
+// L2 (keep_permille)
+#define NBG_L2_KEEP 30
 #endif
 
 namespace {
@@ -122,12 +124,21 @@ struct MixArgs {
     uint32_t keep_pm;  // per mille of each block's matrix stream kept in L2
 };
 
+// Whether the matrix of a block's slice `at` stays in L2 between iterations:
+// keep_pm / 1000 of the slices, spread evenly.  With the first ones kept,
+// DRAM had nothing to do while every warp worked on them (1M-dof ghost form:
+// 33.8 against 34.2 us per iteration).
+__device__ __forceinline__ bool kept(const MixArgs& a, uint32_t at) {
+    return (at + 1) * a.keep_pm / 1000u != at * a.keep_pm / 1000u;
+}
+
 // One system of a launch: its slices, its blocks and its synchronisation.
 struct Group {
     double* part;  // L1 [0,K), L2 [K,3K), init/update [3K,6K), K = pstride
     unsigned* bar;
     int* status;
     double* res;              // niter, updates, status, rr64, bb, b.u
+    unsigned char* sums;      // words of the two fixed-point sums, 2 kExactBytes
     uint32_t s_begin, s_end;  // slices
     uint32_t g_base, g_size;  // blocks [g_base, g_base + g_size) of the launch
     uint32_t pstride;
@@ -186,12 +197,13 @@ struct MixScalars {
     // A reliable update's {|r|^2, r.z, r.p} (FP64), r the recomputed residual
     // and p the last direction: 2 stop, else 0 with beta.  The recursive
     // residual was orthogonal to p, the recomputed one is only up to the
-    // rounding of b - A u, so the next step's numerator is r.(z + beta p), not
-    // r.z: near the FP64 floor of a system the difference is no longer small,
-    // and with r.z the error stayed in every later step until the iteration
-    // diverged (the 20,000-point T3 L-shape at relres 8e-12: 36 after 40,000
-    // iterations).
-    __device__ __forceinline__ int replaced(const double (&t)[3], uint32_t max_iter, FF& beta) {
+    // rounding of b - A u.  Near the FP64 floor of a system r.(z + beta p)
+    // then differs from r.z, and with r.z as the next step's numerator the
+    // error stayed in every later step until the iteration diverged (the
+    // 20,000-point T3 L-shape at relres 8e-12: 36 after 40,000 iterations).
+    // From a relative difference of `least` on the step takes r.(z + beta p).
+    __device__ __forceinline__ int replaced(const double (&t)[3], uint32_t max_iter, FF& beta,
+                                            float least = 0.f) {
         rr64 = t[0];
         rmax2 = (float)rr64;
         nupd++;
@@ -200,12 +212,12 @@ struct MixScalars {
         if (!stop) {
             const FF rzn = ff_from_double(t[1]);
             beta = ff_div(rzn, rz);
-            const FF rp = ff_add(rzn, ff_mul(beta, ff_from_double(t[2])));
-            if (rp.hi > 0.1f * rzn.hi) {
-                rz = rp;
-            } else {  // p points uphill: start again from z
-                beta = FF{0.f, 0.f};
-                rz = rzn;
+            rz = rzn;
+            const FF off = ff_mul(beta, ff_from_double(t[2]));
+            if (!(fabsf(off.hi) <= least * rzn.hi)) {
+                const FF rp = ff_add(rzn, off);
+                if (rp.hi > 0.1f * rzn.hi) rz = rp;
+                else beta = FF{0.f, 0.f};  // p points uphill: start again from z
             }
         }
         return stop ? 2 : 0;
@@ -336,6 +348,80 @@ __device__ __forceinline__ void true_residual(const MixArgs& a, const Own& o, ui
     }
 }
 
+// The two sums of an iteration, in fixed point (allreduce.cuh; 1M-dof ghost
+// form 31.6 us per iteration against 32.9 with block sums, a counting barrier
+// and the partials' loads behind it), with kFence
+// also as a barrier for the vectors in global memory; where a window does not
+// serve, by partials and a barrier (`sync`).  finish(sums ...) runs in thread 0.
+// Nonzero return: stop.  Both forms of the single-system solver use it, with
+// the same values per thread, so they get the same bits.
+struct MixSums {
+    int sh[kSumShared];
+    ExactSum pw, rz;
+    float scale[3];  // windows of p.w, r.z, |r|^2
+    int again;
+
+    __device__ __forceinline__ void init(unsigned char* words) {  // by one thread
+        pw.init(words);
+        rz.init(words + kExactBytes);
+        scale[0] = scale[1] = scale[2] = 0.f;
+    }
+};
+
+struct NoMixSums {
+    float scale[3];
+};
+
+template <int NV, bool kFence, class Sync, class Finish>
+__device__ __forceinline__ int mixed_sum(MixSums& m, ExactSum& site, int first, FF (&v)[NV],
+                                         const Group& g, uint32_t rank, float2* ffred,
+                                         float2* part, Sync sync, Finish finish) {
+    float scale[NV];
+    int window[NV];
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+        scale[k] = m.scale[first + k];
+        window[k] = window_exponent(scale[k]);
+    }
+    exact_begin<NV>(v, scale, m.sh);
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        long long x;
+        int e;
+        const int st = site.sum<NV, kFence>(m.sh, blockDim.x >> 5, g.g_size, g.status, window, x, e);
+        FF t[NV];
+        const FF mine = exact_ff(x, e);
+#pragma unroll
+        for (int k = 0; k < NV; k++)
+            t[k] = {__shfl_sync(0xffffffffu, mine.hi, k), __shfl_sync(0xffffffffu, mine.lo, k)};
+        if (threadIdx.x == 0) {
+            m.again = st;
+            if (!st) {
+#pragma unroll
+                for (int k = 0; k < NV; k++) m.scale[first + k] = window_scale(t[k].hi);
+                finish(t);
+            }
+        }
+    }
+    __syncthreads();
+    if (m.again) {
+        if (m.again == 2) return 1;
+#pragma unroll
+        for (int k = 0; k < NV; k++) v[k] = fast_two_sum(v[k].hi, v[k].lo);
+        group_publish_ff<NV>(v, ffred, part, rank);
+        if (sync()) return 1;
+        FF t[NV];
+        group_reduce0_ff<NV>(part, g.g_size, t);
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int k = 0; k < NV; k++) m.scale[first + k] = window_scale(t[k].hi);
+            finish(t);
+        }
+        __syncthreads();
+    }
+    return 0;
+}
+
 // The solver of one system on the blocks [g_base, g_base + g_size) of the
 // launch: its own slices, group barrier, partial sums and result.  The
 // scalar recurrences (step lengths, residual norms, stopping and update
@@ -343,8 +429,12 @@ __device__ __forceinline__ void true_residual(const MixArgs& a, const Own& o, ui
 // shared memory as FP32 pairs and flags.
 template <bool kRes, int kThreads>
 __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, unsigned char* smem) {
-    // batched launches give each system at most a few dozen blocks
+    // with resident rows the single-system launch sums in fixed point, as the
+    // ghost-node form; rows in global memory leave it bound by DRAM, and
+    // batched launches give each system a few blocks: by partials there
+    constexpr bool kExact = kThreads == kMixThreads && kRes;
     constexpr int kRB = kThreads == kMixThreads ? kReduceBatch : 1;
+    __shared__ std::conditional_t<kExact, MixSums, NoMixSums> ms;
     __shared__ double red[3 * 32];
     float2* const ffred = reinterpret_cast<float2*>(red);
     __shared__ float s_alpha[2], s_beta[2];
@@ -367,7 +457,10 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
     // 4.07 s; the 96-system batch: 1.43 against 1.36 s)
     auto sync = [&]() { return grid_barrier(g.bar, G, rank, g.status); };
 
-    if (threadIdx.x == 0) sc.clear();
+    if (threadIdx.x == 0) {
+        sc.clear();
+        if constexpr (kExact) ms.init(g.sums);
+    }
     {   // init: own copy of 1/Aii, x = 0, r = b - A u (FP64), p = z
         const float2* __restrict__ gdv = reinterpret_cast<const float2*>(a.A.dinv32);
         for (uint32_t s = s0 + warp; s < s1; s += nw) {
@@ -388,7 +481,11 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
     {
         double t[3];
         group_reduce0<3>(part2, G, t);
-        if (threadIdx.x == 0) s_flag = sc.start(t, a);
+        if (threadIdx.x == 0) {
+            s_flag = sc.start(t, a);
+            ms.scale[1] = window_scale(sc.rz.hi);
+            ms.scale[2] = window_scale((float)sc.rr64);
+        }
         __syncthreads();
     }
     while (s_flag != 2) {
@@ -402,8 +499,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
                 // a slice's rows past Nn are padding: skip them whole (both lanes)
                 if (s * 32 + ((h & 1) << 4) >= Nn) continue;
                 FF y0, y1;
-                // the first keep_pm / 1000 of this block's slices stay in L2
-                const uint64_t pol = l2_policy((s - s0) * 1000u < a.keep_pm * (s1 - s0));
+                const uint64_t pol = l2_policy(kept(a, s - s0));
                 spmv_half_split(a, s, r, par, i < Nn, pol, y0, y1);
                 if (par || i >= Nn) continue;
                 o.w[li] = make_float4(y0.hi, y1.hi, y0.lo, y1.lo);
@@ -411,19 +507,25 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
                 pw.fma2(p.x, p.z, y0.hi, y0.lo);
                 pw.fma2(p.y, p.w, y1.hi, y1.lo);
             }
-            FF v[1] = {pw.result()};
-            group_publish_ff<1>(v, ffred, reinterpret_cast<float2*>(part0), rank);
-        }
-        if (sync()) goto done;
-        {
-            FF pw[1];
-            group_reduce0_ff<1, kRB>(reinterpret_cast<const float2*>(part0), G, pw);
-            if (threadIdx.x == 0) {
-                const FF al = sc.alpha(pw[0]);
+            auto finish = [&](const FF (&pws)[1]) {
+                const FF al = sc.alpha(pws[0]);
                 s_alpha[0] = al.hi;
                 s_alpha[1] = al.lo;
+            };
+            if constexpr (kExact) {
+                FF v[1] = {{pw.s, pw.c}};
+                if (mixed_sum<1, true>(ms, ms.pw, 0, v, g, rank, ffred, reinterpret_cast<float2*>(part0),
+                                 sync, finish))
+                    goto done;
+            } else {
+                FF v[1] = {pw.result()};
+                group_publish_ff<1>(v, ffred, reinterpret_cast<float2*>(part0), rank);
+                if (sync()) goto done;
+                FF t[1];
+                group_reduce0_ff<1, kRB>(reinterpret_cast<const float2*>(part0), G, t);
+                if (threadIdx.x == 0) finish(t);
+                __syncthreads();
             }
-            __syncthreads();
         }
         {   // L2: x += alpha p, r -= alpha w, z = r / Aii (own rows only)
             const FF alpha = {s_alpha[0], s_alpha[1]};
@@ -446,22 +548,28 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
                 rrk.fma2(r0.hi, r0.lo, r0.hi, r0.lo);
                 rrk.fma2(r1.hi, r1.lo, r1.hi, r1.lo);
             }
-            FF v[2] = {rzk.result(), rrk.result()};
-            group_publish_ff<2>(v, ffred, reinterpret_cast<float2*>(part1), rank);
-        }
-        if (sync()) goto done;
-        {
-            FF t2[2];
-            group_reduce0_ff<2, kRB>(reinterpret_cast<const float2*>(part1), G, t2);
-            if (threadIdx.x == 0) {
+            auto finish = [&](const FF (&t2)[2]) {
                 FF be;
                 s_flag = sc.step(t2[0], t2[1], a.max_iter, be);
                 if (!s_flag) {
                     s_beta[0] = be.hi;
                     s_beta[1] = be.lo;
                 }
+            };
+            if constexpr (kExact) {
+                FF v[2] = {{rzk.s, rzk.c}, {rrk.s, rrk.c}};
+                if (mixed_sum<2, true>(ms, ms.rz, 1, v, g, rank, ffred, reinterpret_cast<float2*>(part1),
+                                 sync, finish))
+                    goto done;
+            } else {
+                FF v[2] = {rzk.result(), rrk.result()};
+                group_publish_ff<2>(v, ffred, reinterpret_cast<float2*>(part1), rank);
+                if (sync()) goto done;
+                FF t[2];
+                group_reduce0_ff<2, kRB>(reinterpret_cast<const float2*>(part1), G, t);
+                if (threadIdx.x == 0) finish(t);
+                __syncthreads();
             }
-            __syncthreads();
         }
         if (s_flag) {
             // reliable update: u += x in FP64, then r = b - A u in FP64
@@ -488,7 +596,8 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
             group_reduce0<3>(part2, G, tt);
             if (threadIdx.x == 0) {
                 FF be;
-                s_flag = sc.replaced(tt, a.max_iter, be);
+                // rows in global memory: the large systems, far from their floor
+                s_flag = sc.replaced(tt, a.max_iter, be, kRes ? 0.f : 1e-7f);
                 if (!s_flag) {
                     s_beta[0] = be.hi;
                     s_beta[1] = be.lo;
@@ -575,6 +684,11 @@ uint32_t keep_permille(const nbg_bsr_t& A, double bytes_per_entry = 32.0) {
         return 0;
     const double stream = bytes_per_entry * (double)A.n_entries;
     const double budget = l2 * (NBG_L2_KEEP / 100.0);
+    // a stream of more than twice the L2 gains less from the kept part than
+    // its vectors lose (us per iteration without and with: q4 with 2.1M dof
+    // 80.0 and 86.4, T3 with 2.6M dof 99.4 and 106.6, at 1.6 times the L2
+    // 53.8 and 52.2)
+    if (stream > 2.0 * l2) return 0;
     if (stream <= 0.0 || budget >= stream) return 1000;
     return (uint32_t)(1000.0 * budget / stream);
 }
@@ -604,7 +718,7 @@ size_t mixed_bytes(uint32_t N) { return mixed_core_bytes(N) + perm_tail_bytes(N)
 
 // The mixed solver's SpMV operator as its own launch: w = A p with the split
 // matrix and float-float p, two lanes per node row, the solver's L2 policy
-// (the first keep_pm / 1000 of each block's slices evict_last).  One block per
+// (keep_pm / 1000 of each block's slices evict_last).  One block per
 // SM, slices split evenly, as in the solver.
 __global__ void __launch_bounds__(kMixThreads, kMixMinBlocks)
     k_spmv_mixed(MixArgs a, float2* __restrict__ wh, float2* __restrict__ wl) {
@@ -617,7 +731,7 @@ __global__ void __launch_bounds__(kMixThreads, kMixMinBlocks)
         const uint32_t i = s * 32 + r;
         if (s * 32 + ((h & 1) << 4) >= a.A.Nn) continue;
         FF y0, y1;
-        const uint64_t pol = l2_policy((s - s0) * 1000u < a.keep_pm * (s1 - s0));
+        const uint64_t pol = l2_policy(kept(a, s - s0));
         spmv_half_split<true>(a, s, r, par, i < a.A.Nn, pol, y0, y1);
         if (par || i >= a.A.Nn) continue;
         wh[i] = make_float2(y0.hi, y1.hi);
@@ -683,15 +797,19 @@ __device__ __forceinline__ void spmv_half_local(const MixArgs& a, const uint16_t
     y1 = t[1];
 }
 
-// The ghost form keeps r and x in global memory (the workspace's r and x
-// rows).
-__device__ __forceinline__ float4* ghost_r(const MixArgs& a) { return a.r4; }
+// The ghost form keeps r and x in global memory (the workspace's x rows; r in
+// its r and A p rows by turns: L2 reads one and writes the other, so that no
+// block overwrites a row that another may still be reading as a ghost, and
+// the sum between the two needs no fence).
+__device__ __forceinline__ float4* ghost_r(const MixArgs& a, uint32_t turn) {
+    return turn & 1 ? a.w4 : a.r4;
+}
 __device__ __forceinline__ float4* ghost_x(const MixArgs& a) { return a.x4; }
 
 // true_residual for the ghost form: r (float-float) to global memory, where
 // the owner keeps it and the blocks that hold this row as a ghost read it.
 template <int kThreads>
-__device__ __forceinline__ void true_residual_ghost(const MixArgs& a, float4* P,
+__device__ __forceinline__ void true_residual_ghost(const MixArgs& a, float4* r4, float4* P,
                                                     uint32_t s0, uint32_t s1, double& rr,
                                                     FFAcc& rz, double* bb, double* rp,
                                                     bool set_p) {
@@ -700,7 +818,6 @@ __device__ __forceinline__ void true_residual_ghost(const MixArgs& a, float4* P,
     const double2* __restrict__ u = reinterpret_cast<const double2*>(a.u);
     const double2* __restrict__ b = reinterpret_cast<const double2*>(a.b);
     const float2* __restrict__ dinv = reinterpret_cast<const float2*>(a.A.dinv32);
-    float4* __restrict__ r4 = ghost_r(a);
     for (uint32_t s = s0 + warp; s < s1; s += nw) {
         const uint32_t i = s * 32 + lane, li = i - s0 * 32;
         if (i >= a.A.Nn) continue;
@@ -728,6 +845,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
     __shared__ float s_alpha[2], s_beta[2];
     __shared__ int s_flag;  // 0 iterate, 1 reliable update, 2 stop
     __shared__ MixScalars sc;  // thread 0 only
+    __shared__ MixSums ms;
     const unsigned G = g.g_size;
     const uint32_t rank = blockIdx.x - g.g_base;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -742,7 +860,8 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
     // slice offsets of this block, indexed by s - s0
     uint32_t* const SO = NBG_MIXED_SO_SMEM ? GID + gh.gcap
                                            : const_cast<uint32_t*>(a.A.slice_off) + s0;
-    float4* __restrict__ r4 = ghost_r(a);
+    float4* r4 = ghost_r(a, 0);  // the current residual
+    uint32_t turn = 0;
     float4* __restrict__ x4 = ghost_x(a);
     const float2* __restrict__ dinv = reinterpret_cast<const float2*>(a.A.dinv32);
     double* const part0 = g.part;
@@ -755,7 +874,10 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
     auto sync = [&]() { return grid_barrier(g.bar, G, rank, g.status); };
 #endif
 
-    if (tid == 0) sc.clear();
+    if (tid == 0) {
+        sc.clear();
+        ms.init(g.sums);
+    }
     for (uint32_t j = tid; j < ng; j += kThreads) GID[j] = gh.ids[(size_t)rank * kGhostMax + j];
     if (NBG_MIXED_SO_SMEM)
         for (uint32_t j = tid; j <= s1 - s0; j += kThreads) SO[j] = a.A.slice_off[s0 + j];
@@ -767,7 +889,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
         }
         double rrl = 0.0, bbl = 0.0;
         FFAcc rzk{0.f, 0.f};
-        true_residual_ghost<kThreads>(a, P, s0, s1, rrl, rzk, &bbl, nullptr, true);
+        true_residual_ghost<kThreads>(a, r4, P, s0, s1, rrl, rzk, &bbl, nullptr, true);
         const FF t = rzk.result();
         double v[3] = {rrl, bbl, (double)t.hi + (double)t.lo};
         group_publish<3>(v, red, part2, rank);
@@ -776,7 +898,11 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
     {
         double t[3];
         group_reduce0<3>(part2, G, t);
-        if (tid == 0) s_flag = sc.start(t, a);
+        if (tid == 0) {
+            s_flag = sc.start(t, a);
+            ms.scale[1] = window_scale(sc.rz.hi);
+            ms.scale[2] = window_scale((float)sc.rr64);
+        }
         // ghosts start as their owners' p = z
         for (uint32_t j = tid; j < ng; j += kThreads) {
             const uint32_t c = GID[j];
@@ -796,7 +922,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
                 const uint32_t i = s * 32 + r, li = i - s0 * 32;
                 if (s * 32 + ((h & 1) << 4) >= Nn) continue;
                 FF y0, y1;
-                const uint64_t pol = l2_policy((s - s0) * 1000u < a.keep_pm * (s1 - s0));
+                const uint64_t pol = l2_policy(kept(a, s - s0));
                 spmv_half_local(a, gh.lcol, P, SO, s - s0, r, par, i < Nn, pol, y0, y1);
                 if (par || i >= Nn) continue;
                 W[li] = make_float4(y0.hi, y1.hi, y0.lo, y1.lo);
@@ -804,23 +930,19 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
                 pw.fma2(p.x, p.z, y0.hi, y0.lo);
                 pw.fma2(p.y, p.w, y1.hi, y1.lo);
             }
-            FF v[1] = {pw.result()};
-            group_publish_ff<1>(v, ffred, reinterpret_cast<float2*>(part0), rank);
-        }
-        if (sync()) goto done;
-        {
-            FF pw[1];
-            group_reduce0_ff<1>(reinterpret_cast<const float2*>(part0), G, pw);
-            if (tid == 0) {
-                const FF al = sc.alpha(pw[0]);
-                s_alpha[0] = al.hi;
-                s_alpha[1] = al.lo;
-            }
-            __syncthreads();
+            FF v[1] = {{pw.s, pw.c}};
+            if (mixed_sum<1, false>(ms, ms.pw, 0, v, g, rank, ffred, reinterpret_cast<float2*>(part0), sync,
+                             [&](const FF (&pws)[1]) {
+                                 const FF al = sc.alpha(pws[0]);
+                                 s_alpha[0] = al.hi;
+                                 s_alpha[1] = al.lo;
+                             }))
+                goto done;
         }
         {   // L2: x += alpha p, r -= alpha w, z = r / Aii; r published
             const FF alpha = {s_alpha[0], s_alpha[1]};
             FFAcc rzk{0.f, 0.f}, rrk{0.f, 0.f};
+            float4* const rnew = ghost_r(a, ++turn);
             // both dofs of a row at once on the packed FP32x2 instructions
             // (the same roundings as the global-gather form's scalar code)
             const FF2 alpha2 = ff2_bcast(alpha);
@@ -833,7 +955,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
                 x4[i] = make_float4(x.hi.x, x.hi.y, x.lo.x, x.lo.y);
                 const FF2 aw = ff2_mul(alpha2, lohi(W[li]));
                 const FF2 r = ff2_add(lohi(ro), {f2neg(aw.hi), f2neg(aw.lo)});
-                r4[i] = make_float4(r.hi.x, r.hi.y, r.lo.x, r.lo.y);
+                rnew[i] = make_float4(r.hi.x, r.hi.y, r.lo.x, r.lo.y);
                 const FF2 z = ff2_mulf(r, di);
                 rzk.fma2(r.hi.x, r.lo.x, z.hi.x, z.lo.x);
                 rzk.fma2(r.hi.y, r.lo.y, z.hi.y, z.lo.y);
@@ -859,22 +981,18 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
                 row(iA, xA, rA, dA);
                 if (vB) row(iB, xB, rB, dB);
             }
-            FF v[2] = {rzk.result(), rrk.result()};
-            group_publish_ff<2>(v, ffred, reinterpret_cast<float2*>(part1), rank);
-        }
-        if (sync()) goto done;
-        {
-            FF t2[2];
-            group_reduce0_ff<2>(reinterpret_cast<const float2*>(part1), G, t2);
-            if (tid == 0) {
-                FF be;
-                s_flag = sc.step(t2[0], t2[1], a.max_iter, be);
-                if (!s_flag) {
-                    s_beta[0] = be.hi;
-                    s_beta[1] = be.lo;
-                }
-            }
-            __syncthreads();
+            r4 = rnew;
+            FF v[2] = {{rzk.s, rzk.c}, {rrk.s, rrk.c}};
+            if (mixed_sum<2, true>(ms, ms.rz, 1, v, g, rank, ffred, reinterpret_cast<float2*>(part1), sync,
+                             [&](const FF (&t2)[2]) {
+                                 FF be;
+                                 s_flag = sc.step(t2[0], t2[1], a.max_iter, be);
+                                 if (!s_flag) {
+                                     s_beta[0] = be.hi;
+                                     s_beta[1] = be.lo;
+                                 }
+                             }))
+                goto done;
         }
         if (s_flag) {
             // reliable update: u += x in FP64, then r = b - A u in FP64
@@ -892,7 +1010,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
             if (sync()) goto done;
             double rrl = 0.0, rpl = 0.0;
             FFAcc rzk{0.f, 0.f};
-            true_residual_ghost<kThreads>(a, P, s0, s1, rrl, rzk, nullptr, &rpl, false);
+            true_residual_ghost<kThreads>(a, r4, P, s0, s1, rrl, rzk, nullptr, &rpl, false);
             const FF t = rzk.result();
             double v[3] = {rrl, (double)t.hi + (double)t.lo, rpl};
             group_publish<3>(v, red, part2, rank);
@@ -1119,6 +1237,7 @@ extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint
     g.bar = (unsigned*)tail;
     g.status = (int*)(tail + 256);
     g.res = (double*)(tail + 512);
+    g.sums = (unsigned char*)tail + 3 * 256 + kArBytes;
     a.max_iter = max_iter;
     a.tol = tol;
     a.delta = delta;
@@ -1351,7 +1470,10 @@ int batch_plan(nbg_mixed_batch* m, double gamma) {
     a.tol = m->tol;
     a.delta = m->delta;
     a.flags = m->flags;
-    a.keep_pm = keep_permille(m->A);
+    // all of a batch's matrix or nothing: a system reads its part again only
+    // after every other system's (24 systems, 252 MB: 337 ms with none kept,
+    // 351 with a fifth; 12 systems, 41 MB: 33.2 ms with all, 34.2 with none)
+    a.keep_pm = keep_permille(m->A) == 1000 ? 1000 : 0;
     a.resident = dyn > 0;
     std::vector<Group> groups(n);
     std::vector<uint32_t> map(G);
@@ -1364,6 +1486,7 @@ int batch_plan(nbg_mixed_batch* m, double gamma) {
         g.bar = (unsigned*)(m->d_state + i * kStateStride);
         g.status = (int*)(m->d_state + i * kStateStride + 128);
         g.res = m->d_res + i * kResStride;
+        g.sums = nullptr;
         g.s_begin = m->slice_ptr[i];
         g.s_end = m->slice_ptr[i + 1];
         g.g_base = gb;
