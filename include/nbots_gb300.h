@@ -344,7 +344,7 @@ int nbg_cg_mixed(const nbg_bsr_t *A, const double *b, double *x, uint32_t max_it
  * blocks, barrier, reductions and stopping test.  A launch (x = 0, the
  * solve, then the optional SIMP compliance sensitivities with a = b = x) is
  * one CUDA graph replayed on `stream`.  Blocks are shared out in
- * proportion to slices^gamma (nbg_mixed_batch_plan, gamma 1 at creation);
+ * proportion to slices^gamma (nbg_mixed_batch_plan, gamma 1.5 at creation);
  * nbg_mixed_batch_tune times one launch per candidate gamma and keeps the
  * fastest.  Every system needs a co-resident block: n_sys is at most the
  * launch's resident block count.  No counterpart in nbots. */

@@ -1605,7 +1605,12 @@ extern "C" int nbg_mixed_batch_create(nbg_mixed_batch_t** out, const nbg_bsr_t* 
     m->d_groups = (Group*)p;
     p += align256((size_t)n_sys * sizeof(Group));
     m->d_map = (uint32_t*)p;
-    int rc = batch_plan(m, 1.0);
+    // weights slices^1.5: CG's iterations grow with a mesh's length, so with
+    // shares in proportion to the slices the small systems finish early and
+    // their blocks idle (24 systems of 64 to 512 elements' length: 377 ms at
+    // gamma 0.75, 332 at 1, 299 at 1.25, 281 at 1.5, 345 at 1.75; 20 of 96 to
+    // 384: 210, 198, 193, 184, 185)
+    int rc = batch_plan(m, 1.5);
     if (rc != NBG_OK) {
         nbg_mixed_batch_destroy(m);
         return rc;
