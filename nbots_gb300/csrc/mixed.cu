@@ -99,16 +99,6 @@ constexpr int kUnroll = NBG_MIXED_UNROLL;
 
 namespace {
 
-// 1/Aii in shared memory too, or read from global memory (L2) when the
-// shared memory is better left to the L1 cache of the SpMV's gathers
-#ifndef NBG_MIXED_DV_SHARED
-#define NBG_MIXED_DV_SHARED 0
-#endif
-constexpr bool kDvShared = NBG_MIXED_DV_SHARED;
-// own-row bytes per node: p, x, r, A p (16 B each) and 1/Aii (8 B, when
-// shared)
-constexpr size_t kOwnNodeBytes = 64 + (kDvShared ? 8 : 0);
-
 struct MixArgs {
     nbg_bsr_t A;
     const double* b;
@@ -279,33 +269,30 @@ __device__ __forceinline__ void spmv_half_split(const MixArgs& a, uint32_t s, ui
     y1 = t[1];
 }
 
-// Own-row vectors of this block, indexed by local node row
-// (i - 32 * s0): shared memory when they fit, else the global workspace.
+// Own-row vectors of this block, indexed by local node row (i - 32 * s0):
+// those that fit in shared memory, the others in the global workspace.  kOwn:
+// 3 all four, 2 A p and r, 1 A p, 0 none.  Past level 3 the systems are larger
+// than L2 and the iteration is bound by DRAM, to which a vector in global
+// memory adds its reads and writes, 32 B per node row and iteration each for
+// A p and r: 1.28e6 T3 nodes, 500 iterations, 50.4 -> 47.5 ms at level 1
+// instead of 0; 24 batched systems, 252 MB, 281 -> 277.5 ms at level 2.
 struct Own {
     float4 *p, *x, *r, *w;  // {hi, hi, lo, lo}
-    float2* dv;
+    const float2* dv;
 };
+constexpr size_t own_node_bytes(int own) { return own == 3 ? 64 : 16 * (size_t)own; }
 
-template <bool kRes>
+template <int kOwn>
 __device__ __forceinline__ Own own_vectors(const MixArgs& a, unsigned char* smem, uint32_t s0,
                                            uint32_t nrows) {
     Own o;
     const size_t base = (size_t)s0 * 32;
-    if (kRes) {
-        o.p = reinterpret_cast<float4*>(smem);
-        o.x = o.p + nrows;
-        o.r = o.p + 2 * nrows;
-        o.w = o.p + 3 * nrows;
-        o.dv = kDvShared ? reinterpret_cast<float2*>(o.p + 4 * nrows)
-                         : const_cast<float2*>(reinterpret_cast<const float2*>(a.A.dinv32)) +
-                               base;
-    } else {
-        o.p = a.p + base;
-        o.x = a.x4 + base;
-        o.r = a.r4 + base;
-        o.w = a.w4 + base;
-        o.dv = const_cast<float2*>(reinterpret_cast<const float2*>(a.A.dinv32)) + base;
-    }
+    float4* const sh = reinterpret_cast<float4*>(smem);
+    o.p = kOwn == 3 ? sh + 2 * nrows : a.p + base;
+    o.x = kOwn == 3 ? sh + 3 * nrows : a.x4 + base;
+    o.r = kOwn >= 2 ? sh + nrows : a.r4 + base;
+    o.w = kOwn >= 1 ? sh : a.w4 + base;
+    o.dv = reinterpret_cast<const float2*>(a.A.dinv32) + base;
     return o;
 }
 
@@ -427,8 +414,9 @@ __device__ __forceinline__ int mixed_sum(MixSums& m, ExactSum& site, int first, 
 // scalar recurrences (step lengths, residual norms, stopping and update
 // decisions) run in thread 0 (MixScalars) and reach the block through
 // shared memory as FP32 pairs and flags.
-template <bool kRes, int kThreads>
+template <int kOwn, int kThreads>
 __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, unsigned char* smem) {
+    constexpr bool kRes = kOwn == 3;
     // with resident rows the single-system launch sums in fixed point, as the
     // ghost-node form; rows in global memory leave it bound by DRAM, and
     // batched launches give each system a few blocks: by partials there
@@ -447,7 +435,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
     uint32_t s0, s1;
     group_slice_range(g.s_begin, g.s_end, rank, G, s0, s1);
     const uint32_t Nn = a.A.Nn;
-    const Own o = own_vectors<kRes>(a, smem, s0, (s1 - s0) * 32);
+    const Own o = own_vectors<kOwn>(a, smem, s0, (s1 - s0) * 32);
     float4* __restrict__ gp = a.p;
     double* const part0 = g.part;
     double* const part1 = g.part + g.pstride;
@@ -461,13 +449,10 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
         sc.clear();
         if constexpr (kExact) ms.init(g.sums);
     }
-    {   // init: own copy of 1/Aii, x = 0, r = b - A u (FP64), p = z
-        const float2* __restrict__ gdv = reinterpret_cast<const float2*>(a.A.dinv32);
+    {   // init: x = 0, r = b - A u (FP64), p = z
         for (uint32_t s = s0 + warp; s < s1; s += nw) {
             const uint32_t i = s * 32 + lane, li = i - s0 * 32;
-            if (i >= Nn) continue;
-            if (kRes && kDvShared) o.dv[li] = gdv[i];
-            o.x[li] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i < Nn) o.x[li] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
         __syncwarp();
         double rrl = 0.0, bbl = 0.0;
@@ -651,18 +636,18 @@ done:
     }
 }
 
-// kRes: the block's own-row vectors live in dynamic shared memory (known at
-// compile time, so their addresses are 32-bit shared ones).
-template <bool kRes>
+// kOwn: the own-row vectors in dynamic shared memory (known at compile time,
+// so their addresses are 32-bit shared ones).
+template <int kOwn>
 __global__ void __launch_bounds__(kMixThreads, kMixMinBlocks) k_cg_mixed(MixArgs a,
                                                                                 Group g) {
     extern __shared__ __align__(16) unsigned char smem[];
-    mixed_solve<kRes, kMixThreads>(a, g, smem);
+    mixed_solve<kOwn, kMixThreads>(a, g, smem);
 }
 
 // Many independent systems stored in one block-diagonal layout, in one
 // launch: block b works for system groups[block_of[b]].
-template <bool kRes>
+template <int kOwn>
 __global__ void __launch_bounds__(kBatThreads, kBatMinBlocks)
     k_cg_mixed_many(MixArgs a, const Group* __restrict__ groups,
                     const uint32_t* __restrict__ block_of) {
@@ -670,7 +655,7 @@ __global__ void __launch_bounds__(kBatThreads, kBatMinBlocks)
     __shared__ Group sg;
     if (threadIdx.x == 0) sg = groups[block_of[blockIdx.x]];
     __syncthreads();
-    mixed_solve<kRes, kBatThreads>(a, sg, smem);
+    mixed_solve<kOwn, kBatThreads>(a, sg, smem);
 }
 
 // Share of the SpMV's matrix stream (FP32 values, remainders, columns:
@@ -1204,6 +1189,22 @@ int slice_setup(const nbg_bsr_t& A, unsigned G, int threads, char* plan, cudaStr
 }
 }  // namespace
 
+namespace {
+const void* mixed_kernel(int own) {
+    return own == 3 ? (const void*)k_cg_mixed<3>
+         : own == 2 ? (const void*)k_cg_mixed<2>
+         : own == 1 ? (const void*)k_cg_mixed<1>
+                    : (const void*)k_cg_mixed<0>;
+}
+
+const void* batch_kernel(int own) {
+    return own == 3 ? (const void*)k_cg_mixed_many<3>
+         : own == 2 ? (const void*)k_cg_mixed_many<2>
+         : own == 1 ? (const void*)k_cg_mixed_many<1>
+                    : (const void*)k_cg_mixed_many<0>;
+}
+}  // namespace
+
 extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint32_t max_iter,
                             double tol, double delta, unsigned flags, nbg_mixed_result_t* result,
                             void* ws, size_t ws_bytes, void* stream) {
@@ -1265,6 +1266,7 @@ extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const unsigned slice_g = NBG_MIXED_RESIDENT ? slice_grid(A->n_slices, nsm) : 0;
     const void* fn = nullptr;
+    a.resident = 1;
     if (e == cudaSuccess && slice_g) {
         G = slice_g;
         threads = 32 * (int)((A->n_slices + G - 1) / G);
@@ -1281,14 +1283,16 @@ extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint
         if (ghost) fn = (const void*)k_cg_mixed_ghost;
     }
     if (e == cudaSuccess && !fn) {
-        rc = coop_grid_resident((const void*)k_cg_mixed<true>, A->n_slices,
-                                NBG_MIXED_RESIDENT ? kOwnNodeBytes * 32 : 0, &G, &dyn, kMixThreads,
-                                kMixMinBlocks);
-        if (rc == NBG_OK && dyn == 0)
-            rc = coop_grid((const void*)k_cg_mixed<false>, A->n_slices, &G, kMixThreads);
-        fn = dyn > 0 ? (const void*)k_cg_mixed<true> : (const void*)k_cg_mixed<false>;
+        // as many of the own rows' vectors in shared memory as fit, at the
+        // same grid: the rows of a block, and so the sums, are the same
+        for (int own = NBG_MIXED_RESIDENT ? 3 : 0; own >= 0 && rc == NBG_OK && !fn; own--) {
+            fn = mixed_kernel(own);
+            rc = coop_grid_resident(fn, A->n_slices, own_node_bytes(own) * 32, &G, &dyn, kMixThreads,
+                                    kMixMinBlocks);
+            a.resident = own == 3;
+            if (own > 0 && dyn == 0) fn = nullptr;
+        }
     }
-    a.resident = dyn > 0;
     g.s_begin = 0;
     g.s_end = A->n_slices;
     g.g_base = 0;
@@ -1342,6 +1346,7 @@ struct nbg_mixed_batch {
     unsigned char* d_state;
     unsigned G;
     size_t dyn;
+    int own;  // own-row vectors in shared memory (mixed_solve's kOwn)
     // compliance sensitivities after the solve (a = b = x)
     bool sens;
     uint32_t nen, N_elem;
@@ -1420,36 +1425,52 @@ void drop_graph(nbg_mixed_batch* m) {
 
 // Block shares, launch size and the per-system argument table for `gamma`.
 int batch_plan(nbg_mixed_batch* m, double gamma) {
-    const void* fn = (const void*)k_cg_mixed_many<true>;
     int dev = 0, nsm = 0, optin = 0;
     NBG_CHECK(cudaGetDevice(&dev));
     NBG_CHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     NBG_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    cudaFuncAttributes fa;
-    NBG_CHECK(cudaFuncGetAttributes(&fa, fn));
     const uint32_t n = m->n_sys;
     std::vector<uint32_t> bl;
     unsigned G = 0;
     size_t dyn = 0;
-    // own rows in shared memory when every block's rows fit
-    for (int per_sm = kBatMinBlocks; NBG_MIXED_RESIDENT && per_sm >= 1 && !G; --per_sm) {
+    int own = NBG_MIXED_RESIDENT ? 3 : 0;
+    // a launch of per_sm blocks per SM that keeps `own` vectors of its rows in
+    // shared memory, when it fits
+    auto fits = [&](int per_sm) -> int {
+        const void* fn = batch_kernel(own);
+        cudaFuncAttributes fa;
+        NBG_CHECK(cudaFuncGetAttributes(&fa, fn));
         const unsigned total = std::min<unsigned>((unsigned)nsm * per_sm, kMaxBlocks);
-        if (n > total) break;
+        if (n > total) return NBG_OK;
         share_blocks(m->slice_ptr, gamma, total, bl);
-        const size_t bytes = (size_t)max_slices_per_block(m->slice_ptr, bl) * kOwnNodeBytes * 32;
-        if (bytes + fa.sharedSizeBytes > (size_t)optin) continue;
+        const size_t bytes =
+            (size_t)max_slices_per_block(m->slice_ptr, bl) * own_node_bytes(own) * 32;
+        if (bytes + fa.sharedSizeBytes > (size_t)optin) return NBG_OK;
         NBG_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
         int occ = 0;
         NBG_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kBatThreads, bytes));
         unsigned used = 0;
         for (uint32_t v : bl) used += v;
-        if ((unsigned)occ * (unsigned)nsm >= used) {
+        if ((uint64_t)occ * (unsigned)nsm >= used) {
             G = used;
             dyn = bytes;
         }
+        return NBG_OK;
+    };
+    // all own rows in shared memory, with fewer blocks per SM if need be;
+    // else at the full block count as many of the vectors as fit
+    for (int per_sm = kBatMinBlocks; own == 3 && per_sm >= 1 && !G; --per_sm) {
+        const int rc = fits(per_sm);
+        if (rc != NBG_OK) return rc;
+    }
+    while (!G && own > 1) {
+        own--;
+        const int rc = fits(kBatMinBlocks);
+        if (rc != NBG_OK) return rc;
     }
     if (!G) {
-        fn = (const void*)k_cg_mixed_many<false>;
+        own = 0;
+        const void* fn = batch_kernel(0);
         int occ = 0;
         NBG_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kBatThreads, 0));
         const unsigned total = std::min<unsigned>((unsigned)nsm * (unsigned)std::max(occ, 1), kMaxBlocks);
@@ -1474,7 +1495,8 @@ int batch_plan(nbg_mixed_batch* m, double gamma) {
     // after every other system's (24 systems, 252 MB: 337 ms with none kept,
     // 351 with a fifth; 12 systems, 41 MB: 33.2 ms with all, 34.2 with none)
     a.keep_pm = keep_permille(m->A) == 1000 ? 1000 : 0;
-    a.resident = dyn > 0;
+    a.resident = own == 3;
+    m->own = own;
     std::vector<Group> groups(n);
     std::vector<uint32_t> map(G);
     double* part = part_slots(base, m->A.N);
@@ -1521,8 +1543,9 @@ cudaError_t batch_enqueue(nbg_mixed_batch* m, cudaStream_t s) {
     cfg.numAttrs = 1;
     const Group* groups = m->d_groups;
     const uint32_t* map = m->d_map;
-    e = m->args.resident ? cudaLaunchKernelEx(&cfg, k_cg_mixed_many<true>, m->args, groups, map)
-                         : cudaLaunchKernelEx(&cfg, k_cg_mixed_many<false>, m->args, groups, map);
+    MixArgs args = m->args;
+    void* params[] = {&args, &groups, &map};
+    e = cudaLaunchKernelExC(&cfg, batch_kernel(m->own), params);
     if (e != cudaSuccess || !m->sens) return e;
     const int rc = nbg_simp_sensitivity_f64(m->nen, m->N_elem, m->nod, m->conn, m->nu,
                                             m->thickness, m->rho, m->penal, m->E0, m->Emin, m->x,
@@ -1533,8 +1556,8 @@ cudaError_t batch_enqueue(nbg_mixed_batch* m, cudaStream_t s) {
 // The function attribute is shared by every batch in the process: set it
 // to this batch's size before capturing and before each replay.
 int set_smem(const nbg_mixed_batch* m) {
-    if (m->args.resident)
-        NBG_CHECK(cudaFuncSetAttribute((const void*)k_cg_mixed_many<true>,
+    if (m->own)
+        NBG_CHECK(cudaFuncSetAttribute(batch_kernel(m->own),
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m->dyn));
     return NBG_OK;
 }

@@ -1,0 +1,67 @@
+"""The mixed solver's global-gather form at the sizes where fewer of the own
+rows' vectors fit in shared memory: all four, A p and r, A p, none.  After a
+budget of 40 iterations the residual that the recurrence reports is that of
+the oracle's SpMV: each iteration rounds at 2^-47 of |A||p| alpha, up to some
+1e3 |r| while the iterate is far from converged, 40 of them below 1e-9; the
+bound is ten times that."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+BUDGET, RTOL = 40, 1e-8
+
+
+# node rows per SM: 110 and 112 slices of 32, 225 and 228, 451 and 454
+# (2 KiB per slice for all vectors, 1 KiB, 512 B, of 227 KiB per SM)
+@pytest.mark.parametrize("nx,ny", [(799, 667), (799, 681), (1023, 1068), (1023, 1083),
+                                   (1999, 1097), (1999, 1105)])
+def test_single_system(nx, ny):
+    from nbots_gb300 import _lib as L, workloads as W
+    from nbots_gb300.device import DeviceArray
+    from nbots_gb300.fem import FemSystem
+    p = W.cantilever_q4(nx, ny - ny % 2, top_traction=0.01)
+    p.E = W.lognormal_E(p.n_elems, 0.3, 5)
+    s = FemSystem(p)
+    assert s.assemble() == 0
+    s.apply_bcs()
+    lib, A = L.lib(), s.block_layout()
+    n = lib.nbg_cg_mixed_workspace_bytes(s.N)  # without room for a ghost plan
+    ws, u, r = DeviceArray(np.zeros(n, np.uint8)), DeviceArray(np.zeros(s.N)), L.MixedResult()
+    rc = lib.nbg_cg_mixed(C.byref(A), s.dptr(L.FEM_F), u.ptr, BUDGET, 1e-12, 0.1,
+                          L.CG_JACOBI | L.CG_RELATIVE, C.byref(r), ws.ptr, n, None)
+    assert rc == 1 and r.niter == BUDGET
+    assert lib.nbg_cg_mixed_last_form() == (1 if p.n_nodes <= 152 * 111 * 32 else 0)
+    F = s.get(L.FEM_F)
+    res = F - O.spmv(s.get(L.FEM_ROW_PTR), s.get(L.FEM_COL_IDX), s.get(L.FEM_K), u.numpy())
+    rel = np.linalg.norm(res) / np.linalg.norm(F)
+    assert abs(rel - r.relres) <= RTOL * rel
+    s.close()
+
+
+# 3,738 slices per system: 98 per SM (all vectors), 123 (31 per block: two),
+# 221 (56 per block: one), 443 (111 per block: none)
+@pytest.mark.parametrize("count", [4, 5, 9, 18])
+def test_batch(count):
+    from nbots_gb300 import _lib as L, workloads as W
+    from nbots_gb300.batch import Batch
+    p = W.cantilever_q4(600, 198)
+    rho = np.random.Generator(np.random.PCG64(3)).uniform(0.3, 0.7, size=p.n_elems)
+    b = Batch([p] * count)
+    b.assemble_simp([rho] * count, p.nu)
+    b.setup(max_iter=BUDGET, tol=1e-12)
+    b.launch()
+    res, _ = b.results()
+    rp, ci, K, F, u = (b.merged(w) for w in (L.FEM_ROW_PTR, L.FEM_COL_IDX, L.FEM_K, L.FEM_F,
+                                             L.FEM_U))
+    for k in (0, count - 1):
+        assert res[k].niter == BUDGET
+        r0, r1 = 2 * int(b.node_off[k]), 2 * int(b.node_off[k]) + p.n_dof
+        seg = slice(int(rp[r0]), int(rp[r1]))
+        y = O.spmv(rp[r0:r1 + 1] - rp[r0], (ci[seg] - r0).astype(np.uint32), K[seg], u[r0:r1])
+        rel = np.linalg.norm(F[r0:r1] - y) / np.linalg.norm(F[r0:r1])
+        assert abs(rel - res[k].relres) <= RTOL * rel
+    b.close()
