@@ -203,19 +203,13 @@ int ghost_plan(const nbg_bsr_t& A, unsigned G, char* plan, cudaStream_t s, Ghost
     return 1;
 }
 
-// Whether `bytes` of dynamic shared memory let G blocks of `fn` run at once;
-// sets the kernel's limit to them.
+// Whether `bytes` of dynamic shared memory let G blocks of `fn` run at once.
 bool fits_smem(const void* fn, int threads, size_t bytes, unsigned G) {
-    int dev = 0, nsm = 0, optin = 0, occ = 0;
-    cudaFuncAttributes fa;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
-            cudaSuccess ||
-        cudaFuncGetAttributes(&fa, fn) != cudaSuccess || bytes + fa.sharedSizeBytes > (size_t)optin)
-        return false;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) ==
-               cudaSuccess &&
+    int dev = 0, nsm = 0, occ = 0;
+    size_t most = 0;
+    return cudaGetDevice(&dev) == cudaSuccess &&
+           cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+           allow_smem(fn, &most) == cudaSuccess && bytes <= most &&
            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, bytes) ==
                cudaSuccess &&
            (uint64_t)occ * (unsigned)nsm >= G;

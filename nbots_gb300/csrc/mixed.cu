@@ -1425,10 +1425,9 @@ void drop_graph(nbg_mixed_batch* m) {
 
 // Block shares, launch size and the per-system argument table for `gamma`.
 int batch_plan(nbg_mixed_batch* m, double gamma) {
-    int dev = 0, nsm = 0, optin = 0;
+    int dev = 0, nsm = 0;
     NBG_CHECK(cudaGetDevice(&dev));
     NBG_CHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    NBG_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     const uint32_t n = m->n_sys;
     std::vector<uint32_t> bl;
     unsigned G = 0;
@@ -1438,15 +1437,14 @@ int batch_plan(nbg_mixed_batch* m, double gamma) {
     // shared memory, when it fits
     auto fits = [&](int per_sm) -> int {
         const void* fn = batch_kernel(own);
-        cudaFuncAttributes fa;
-        NBG_CHECK(cudaFuncGetAttributes(&fa, fn));
+        size_t most = 0;
+        NBG_CHECK(allow_smem(fn, &most));
         const unsigned total = std::min<unsigned>((unsigned)nsm * per_sm, kMaxBlocks);
         if (n > total) return NBG_OK;
         share_blocks(m->slice_ptr, gamma, total, bl);
         const size_t bytes =
             (size_t)max_slices_per_block(m->slice_ptr, bl) * own_node_bytes(own) * 32;
-        if (bytes + fa.sharedSizeBytes > (size_t)optin) return NBG_OK;
-        NBG_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        if (bytes > most) return NBG_OK;
         int occ = 0;
         NBG_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kBatThreads, bytes));
         unsigned used = 0;
@@ -1553,18 +1551,7 @@ cudaError_t batch_enqueue(nbg_mixed_batch* m, cudaStream_t s) {
     return rc == NBG_OK ? cudaSuccess : cudaErrorLaunchFailure;
 }
 
-// The function attribute is shared by every batch in the process: set it
-// to this batch's size before capturing and before each replay.
-int set_smem(const nbg_mixed_batch* m) {
-    if (m->own)
-        NBG_CHECK(cudaFuncSetAttribute(batch_kernel(m->own),
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m->dyn));
-    return NBG_OK;
-}
-
 int build_graph(nbg_mixed_batch* m) {
-    const int rc = set_smem(m);
-    if (rc != NBG_OK) return rc;
     cudaStream_t cap;
     NBG_CHECK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
     cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
@@ -1687,7 +1674,7 @@ extern "C" int nbg_mixed_batch_set_sensitivity(nbg_mixed_batch_t* m, uint32_t ne
 
 extern "C" int nbg_mixed_batch_launch(nbg_mixed_batch_t* m) {
     if (!m) return NBG_ERR_ARG;
-    const int rc = m->exec ? set_smem(m) : build_graph(m);
+    const int rc = m->exec ? NBG_OK : build_graph(m);
     if (rc != NBG_OK) return rc;
     NBG_CHECK(cudaGraphLaunch(m->exec, m->stream));
     return NBG_OK;

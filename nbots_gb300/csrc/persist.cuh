@@ -314,6 +314,22 @@ inline int coop_grid(const void* fn, uint32_t n_slices, unsigned* G,
     return NBG_OK;
 }
 
+// Lets fn be launched with up to *most bytes of dynamic shared memory, all
+// that its static use leaves.  Always the same value: the attribute is the
+// process's, and a smaller one, set for one launch, would refuse a larger
+// launch that another thread is about to make.
+inline cudaError_t allow_smem(const void* fn, size_t* most) {
+    int dev = 0, optin = 0;
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);
+    if (e != cudaSuccess) return e;
+    *most = (size_t)optin - fa.sharedSizeBytes;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*most);
+}
+
 // Grid of a persistent kernel whose blocks keep `bytes_per_slice` of own-row
 // data per slice in dynamic shared memory: the largest blocks-per-SM count
 // (min_blocks, then fewer) at which every block's slices fit.  *dyn = 0
@@ -322,12 +338,11 @@ inline int coop_grid(const void* fn, uint32_t n_slices, unsigned* G,
 inline int coop_grid_resident(const void* fn, uint32_t n_slices, size_t bytes_per_slice,
                               unsigned* G, size_t* dyn, int threads = kPersistThreads,
                               int min_blocks = kPersistMinBlocks) {
-    int dev = 0, nsm = 0, optin = 0;
+    int dev = 0, nsm = 0;
+    size_t most = 0;
     NBG_CHECK(cudaGetDevice(&dev));
     NBG_CHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    NBG_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    cudaFuncAttributes fa;
-    NBG_CHECK(cudaFuncGetAttributes(&fa, fn));
+    NBG_CHECK(allow_smem(fn, &most));
     const unsigned want = (n_slices + threads / 32 - 1) / (threads / 32);
     for (int per_sm = min_blocks; bytes_per_slice && per_sm >= 1; --per_sm) {
         unsigned g = (unsigned)nsm * (unsigned)per_sm;
@@ -335,9 +350,7 @@ inline int coop_grid_resident(const void* fn, uint32_t n_slices, size_t bytes_pe
         if (g < 1) g = 1;
         const size_t spb = (n_slices + g - 1) / g;
         const size_t bytes = spb * bytes_per_slice;
-        if (bytes + fa.sharedSizeBytes > (size_t)optin) continue;
-        NBG_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)bytes));
+        if (bytes > most) continue;
         int occ = 0;
         NBG_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, bytes));
         if ((unsigned)occ * (unsigned)nsm >= g) {
@@ -347,7 +360,6 @@ inline int coop_grid_resident(const void* fn, uint32_t n_slices, size_t bytes_pe
         }
     }
     *dyn = 0;
-    NBG_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 0));
     return coop_grid(fn, n_slices, G, threads);
 }
 
