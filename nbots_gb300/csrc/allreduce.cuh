@@ -309,6 +309,14 @@ __device__ __forceinline__ void exact_begin(const V (&v)[NV], const W (&window)[
     }
 }
 
+// Named barriers of the whole block (0 is __syncthreads).
+__device__ __forceinline__ void bar_arrive(int id) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(blockDim.x) : "memory");
+}
+__device__ __forceinline__ void bar_sync(int id) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(blockDim.x) : "memory");
+}
+
 // One place in a kernel where sums are taken (in shared memory: only warp 0
 // uses it).
 struct ExactSum {
@@ -325,11 +333,12 @@ struct ExactSum {
     // grid's G <= 255 blocks, value 0 in the even lanes and value 1 in the odd
     // ones (one value: in every lane), as an integer x of 61 bits and an
     // exponent e: x 2^e.  kFence: the sum is also a barrier for the block's
-    // plain loads and stores (release before it, acquire after it).  Returns 0, 1 (outside the window: sum again by records)
-    // or 2 (give up).  Called by one whole warp.
-    template <int NV, bool kFence = false>
+    // plain loads and stores (release before it, acquire after it).  out() is
+    // called when the block's part is on its way.  Returns 0, 1 (outside the
+    // window: sum again by records) or 2 (give up).  Called by one whole warp.
+    template <int NV, bool kFence, class Out>
     __device__ __forceinline__ int sum(const int* sh, uint32_t n_warps, uint32_t G, int* status,
-                                       const int (&window)[NV], long long& x, int& e) {
+                                       const int (&window)[NV], long long& x, int& e, Out out) {
         const uint32_t lane = threadIdx.x & 31;
         constexpr uint32_t kW = NV * kSumWords;
         // lanes 0-15 add the even warps' words, lanes 16-31 the odd ones'
@@ -348,17 +357,20 @@ struct ExactSum {
             const unsigned long long add = (1ull << 56) + (unsigned long long)(mine + (1ll << 32));
             asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(add) : "memory");
         }
+        out();
         PollLimit lim;
         for (;;) {
             bool ok = true;
             if (lane < kW) {
-                asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(d) : "l"(p) : "memory");
+                if (kFence)  // not a fence behind the loop: it would wait for stores too
+                    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(d) : "l"(p) : "memory");
+                else
+                    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(d) : "l"(p) : "memory");
                 ok = ((d - before) >> 56) == G;
             }
             if (__all_sync(0xffffffffu, ok)) break;
             if (__any_sync(0xffffffffu, lim.expired(status))) return 2;
         }
-        if (kFence) __threadfence();
         const long long t = (long long)((d - before) & ((1ull << 56) - 1)) - ((long long)G << 32);
         if (lane < kW) last[h][lane] = d;
         if (lane == 0) half = h ^ 1;
@@ -384,6 +396,11 @@ struct ExactSum {
         x = v << up;
         e = (NV == 2 && k ? window[NV - 1] : window[0]) - 4 * kLimbBits - m - up;
         return __any_sync(0xffffffffu, bad);
+    }
+    template <int NV>
+    __device__ __forceinline__ int sum(const int* sh, uint32_t n_warps, uint32_t G, int* status,
+                                       const int (&window)[NV], long long& x, int& e) {
+        return sum<NV, false>(sh, n_warps, G, status, window, x, e, [] {});
     }
 };
 

@@ -359,10 +359,11 @@ struct NoMixSums {
     float scale[3];
 };
 
-template <int NV, bool kFence, class Sync, class Finish>
+template <int NV, bool kFence, class Sync, class Finish, class Meanwhile>
 __device__ __forceinline__ int mixed_sum(MixSums& m, ExactSum& site, int first, FF (&v)[NV],
                                          const Group& g, uint32_t rank, float2* ffred,
-                                         float2* part, Sync sync, Finish finish) {
+                                         float2* part, Sync sync, Finish finish,
+                                         Meanwhile meanwhile) {
     float scale[NV];
     int window[NV];
 #pragma unroll
@@ -375,7 +376,8 @@ __device__ __forceinline__ int mixed_sum(MixSums& m, ExactSum& site, int first, 
     if (threadIdx.x < 32) {
         long long x;
         int e;
-        const int st = site.sum<NV, kFence>(m.sh, blockDim.x >> 5, g.g_size, g.status, window, x, e);
+        const int st = site.sum<NV, kFence>(m.sh, blockDim.x >> 5, g.g_size, g.status, window, x, e,
+                                            [] { if (kFence) bar_arrive(1); });
         FF t[NV];
         const FF mine = exact_ff(x, e);
 #pragma unroll
@@ -389,6 +391,10 @@ __device__ __forceinline__ int mixed_sum(MixSums& m, ExactSum& site, int first, 
                 finish(t);
             }
         }
+    } else {
+        // memory traffic waits until the fence is over, which would wait for it
+        if (kFence) bar_sync(1);
+        meanwhile();
     }
     __syncthreads();
     if (m.again) {
@@ -500,7 +506,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
             if constexpr (kExact) {
                 FF v[1] = {{pw.s, pw.c}};
                 if (mixed_sum<1, true>(ms, ms.pw, 0, v, g, rank, ffred, reinterpret_cast<float2*>(part0),
-                                 sync, finish))
+                                 sync, finish, [] {}))
                     goto done;
             } else {
                 FF v[1] = {pw.result()};
@@ -544,7 +550,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
             if constexpr (kExact) {
                 FF v[2] = {{rzk.s, rzk.c}, {rrk.s, rrk.c}};
                 if (mixed_sum<2, true>(ms, ms.rz, 1, v, g, rank, ffred, reinterpret_cast<float2*>(part1),
-                                 sync, finish))
+                                 sync, finish, [] {}))
                     goto done;
             } else {
                 FF v[2] = {rzk.result(), rrk.result()};
@@ -743,11 +749,16 @@ __global__ void __launch_bounds__(kMixThreads, kMixMinBlocks)
 // global-gather form bit for bit.  x moves to global memory to leave shared
 // memory to the ghosts.
 //
+// At 1.05M dof an iteration (65 thousand cycles) was two thirds SpMV, at 70 to
+// 78 % of DRAM's rate, then 5 to 6 thousand cycles for each sum, 6.5 for L2 and
+// 4.3 for L3.  So x is updated while warp 0 sums (from when its fence is over:
+// the fence, 2,000 cycles, waits for all the traffic before it), and L2 leaves
+// z in A p's place, so that L3 reads the own rows from shared memory.
+// Microseconds per iteration before and after: 314,000 dof 13.2 and 12.6,
+// 482,000 18.8 and 18.1, 1.05M 31.9 and 30.7, 1.30M 40.4 and 38.9.
+//
 // The plan (ghost lists, local columns) depends on the launch's block
 // partition and is rebuilt by a short kernel at the start of every solve.
-#ifndef NBG_MIXED_SO_SMEM
-#define NBG_MIXED_SO_SMEM 1  // the block's slice offsets in shared memory
-#endif
 // spmv_half_split with local columns and p (own rows and ghosts) in shared
 // memory as float4 {hi of both dofs, lo of both dofs}; the same products and
 // sums in the same order.
@@ -792,12 +803,13 @@ __device__ __forceinline__ float4* ghost_r(const MixArgs& a, uint32_t turn) {
 __device__ __forceinline__ float4* ghost_x(const MixArgs& a) { return a.x4; }
 
 // true_residual for the ghost form: r (float-float) to global memory, where
-// the owner keeps it and the blocks that hold this row as a ghost read it.
+// the owner keeps it and the blocks that hold this row as a ghost read it, z
+// to Z.
 template <int kThreads>
-__device__ __forceinline__ void true_residual_ghost(const MixArgs& a, float4* r4, float4* P,
-                                                    uint32_t s0, uint32_t s1, double& rr,
-                                                    FFAcc& rz, double* bb, double* rp,
-                                                    bool set_p) {
+__device__ __forceinline__ void true_residual_ghost(const MixArgs& a, float4* r4, const float4* P,
+                                                    float4* Z, uint32_t s0, uint32_t s1,
+                                                    double& rr, FFAcc& rz, double* bb,
+                                                    double* rp) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t nw = kThreads / 32;
     const double2* __restrict__ u = reinterpret_cast<const double2*>(a.u);
@@ -818,7 +830,7 @@ __device__ __forceinline__ void true_residual_ghost(const MixArgs& a, float4* r4
         const FF z0 = ff_mulf(f0, di.x), z1 = ff_mulf(f1, di.y);
         rz.fma2(f0.hi, f0.lo, z0.hi, z0.lo);
         rz.fma2(f1.hi, f1.lo, z1.hi, z1.lo);
-        if (set_p) P[li] = make_float4(z0.hi, z1.hi, z0.lo, z1.lo);
+        Z[li] = make_float4(z0.hi, z1.hi, z0.lo, z1.lo);
     }
 }
 
@@ -840,11 +852,10 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
     const uint32_t Nn = a.A.Nn, nslot = (s1 - s0) * 32;
     const uint32_t ng = gh.count[rank];
     float4* const P = reinterpret_cast<float4*>(smem);
-    float4* const W = P + gh.pcap;  // A p of the own rows {hi, hi, lo, lo}
+    float4* const W = P + gh.pcap;  // A p, then z of the own rows {hi, hi, lo, lo}
     uint32_t* const GID = reinterpret_cast<uint32_t*>(W + gh.scap);
     // slice offsets of this block, indexed by s - s0
-    uint32_t* const SO = NBG_MIXED_SO_SMEM ? GID + gh.gcap
-                                           : const_cast<uint32_t*>(a.A.slice_off) + s0;
+    uint32_t* const SO = GID + gh.gcap;
     float4* r4 = ghost_r(a, 0);  // the current residual
     uint32_t turn = 0;
     float4* __restrict__ x4 = ghost_x(a);
@@ -859,13 +870,17 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
     auto sync = [&]() { return grid_barrier(g.bar, G, rank, g.status); };
 #endif
 
+    auto as4 = [](const FF2& v) { return make_float4(v.hi.x, v.hi.y, v.lo.x, v.lo.y); };
+    auto from4 = [](float4 v) -> FF2 {
+        return {make_float2(v.x, v.y), make_float2(v.z, v.w)};
+    };
+
     if (tid == 0) {
         sc.clear();
         ms.init(g.sums);
     }
     for (uint32_t j = tid; j < ng; j += kThreads) GID[j] = gh.ids[(size_t)rank * kGhostMax + j];
-    if (NBG_MIXED_SO_SMEM)
-        for (uint32_t j = tid; j <= s1 - s0; j += kThreads) SO[j] = a.A.slice_off[s0 + j];
+    for (uint32_t j = tid; j <= s1 - s0; j += kThreads) SO[j] = a.A.slice_off[s0 + j];
     {   // init: x = 0, r = b - A u (FP64), own p = z, r published
         for (uint32_t s = s0 + warp; s < s1; s += nw) {
             const uint32_t i = s * 32 + lane;
@@ -874,7 +889,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
         }
         double rrl = 0.0, bbl = 0.0;
         FFAcc rzk{0.f, 0.f};
-        true_residual_ghost<kThreads>(a, r4, P, s0, s1, rrl, rzk, &bbl, nullptr, true);
+        true_residual_ghost<kThreads>(a, r4, P, P, s0, s1, rrl, rzk, &bbl, nullptr);
         const FF t = rzk.result();
         double v[3] = {rrl, bbl, (double)t.hi + (double)t.lo};
         group_publish<3>(v, red, part2, rank);
@@ -921,27 +936,23 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
                                  const FF al = sc.alpha(pws[0]);
                                  s_alpha[0] = al.hi;
                                  s_alpha[1] = al.lo;
-                             }))
+                             }, [] {}))
                 goto done;
         }
-        {   // L2: x += alpha p, r -= alpha w, z = r / Aii; r published
+        {   // L2: r -= alpha w, z = r / Aii; r published; x += alpha p
             const FF alpha = {s_alpha[0], s_alpha[1]};
             FFAcc rzk{0.f, 0.f}, rrk{0.f, 0.f};
             float4* const rnew = ghost_r(a, ++turn);
             // both dofs of a row at once on the packed FP32x2 instructions
             // (the same roundings as the global-gather form's scalar code)
             const FF2 alpha2 = ff2_bcast(alpha);
-            auto lohi = [](float4 v) -> FF2 {
-                return {make_float2(v.x, v.y), make_float2(v.z, v.w)};
-            };
-            auto row = [&](uint32_t i, float4 xo, float4 ro, float2 di) {
+            auto row = [&](uint32_t i, float4 ro, float2 di) {
                 const uint32_t li = i - s0 * 32;
-                const FF2 x = ff2_add(lohi(xo), ff2_mul(alpha2, lohi(P[li])));
-                x4[i] = make_float4(x.hi.x, x.hi.y, x.lo.x, x.lo.y);
-                const FF2 aw = ff2_mul(alpha2, lohi(W[li]));
-                const FF2 r = ff2_add(lohi(ro), {f2neg(aw.hi), f2neg(aw.lo)});
-                rnew[i] = make_float4(r.hi.x, r.hi.y, r.lo.x, r.lo.y);
+                const FF2 aw = ff2_mul(alpha2, from4(W[li]));
+                const FF2 r = ff2_add(from4(ro), {f2neg(aw.hi), f2neg(aw.lo)});
+                rnew[i] = as4(r);
                 const FF2 z = ff2_mulf(r, di);
+                W[li] = as4(z);  // for L3, in place of A p
                 rzk.fma2(r.hi.x, r.lo.x, z.hi.x, z.lo.x);
                 rzk.fma2(r.hi.y, r.lo.y, z.hi.y, z.lo.y);
                 rrk.fma2(r.hi.x, r.lo.x, r.hi.x, r.lo.x);
@@ -954,18 +965,29 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
                 const uint32_t iA = s * 32 + lane, iB = iA + 32 * nw;
                 if (iA >= Nn) continue;
                 const bool vB = s + nw < s1 && iB < Nn;
-                const float4 xA = x4[iA], rA = r4[iA];
+                const float4 rA = r4[iA];
                 const float2 dA = dinv[iA];
-                float4 xB{}, rB{};
+                float4 rB{};
                 float2 dB{};
                 if (vB) {
-                    xB = x4[iB];
                     rB = r4[iB];
                     dB = dinv[iB];
                 }
-                row(iA, xA, rA, dA);
-                if (vB) row(iB, xB, rB, dB);
+                row(iA, rA, dA);
+                if (vB) row(iB, rB, dB);
             }
+            // x += alpha p by the other warps while warp 0 sums: off the
+            // critical path
+            auto update_x = [&]() {
+                const uint32_t step = 32 * (nw - 1);
+                for (uint32_t iA = s0 * 32 + tid - 32; iA < s1 * 32 && iA < Nn; iA += 2 * step) {
+                    const uint32_t iB = iA + step;
+                    const bool vB = iB < s1 * 32 && iB < Nn;
+                    const float4 xA = x4[iA], xB = vB ? x4[iB] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    x4[iA] = as4(ff2_add(from4(xA), ff2_mul(alpha2, from4(P[iA - s0 * 32]))));
+                    if (vB) x4[iB] = as4(ff2_add(from4(xB), ff2_mul(alpha2, from4(P[iB - s0 * 32]))));
+                }
+            };
             r4 = rnew;
             FF v[2] = {{rzk.s, rzk.c}, {rrk.s, rrk.c}};
             if (mixed_sum<2, true>(ms, ms.rz, 1, v, g, rank, ffred, reinterpret_cast<float2*>(part1), sync,
@@ -976,7 +998,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
                                      s_beta[0] = be.hi;
                                      s_beta[1] = be.lo;
                                  }
-                             }))
+                             }, update_x))
                 goto done;
         }
         if (s_flag) {
@@ -995,7 +1017,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
             if (sync()) goto done;
             double rrl = 0.0, rpl = 0.0;
             FFAcc rzk{0.f, 0.f};
-            true_residual_ghost<kThreads>(a, r4, P, s0, s1, rrl, rzk, nullptr, &rpl, false);
+            true_residual_ghost<kThreads>(a, r4, P, W, s0, s1, rrl, rzk, nullptr, &rpl);
             const FF t = rzk.result();
             double v[3] = {rrl, (double)t.hi + (double)t.lo, rpl};
             group_publish<3>(v, red, part2, rank);
@@ -1016,38 +1038,23 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
         {   // L3: p = z + beta p for the own rows and the ghosts (no barrier:
             // every p this block's next SpMV reads is in its shared memory)
             const FF beta = {s_beta[0], s_beta[1]};
-            // p slot l from the row's r (hi, lo) and 1/Aii
             const FF2 beta2 = ff2_bcast(beta);
-            auto pnew = [&](uint32_t l, float4 rv, float2 di) {
-                const float4 p = P[l];
-                const FF2 n = ff2_add(ff2_mulf({make_float2(rv.x, rv.y), make_float2(rv.z, rv.w)}, di),
-                                      ff2_mul(beta2, {make_float2(p.x, p.y), make_float2(p.z, p.w)}));
-                P[l] = make_float4(n.hi.x, n.hi.y, n.lo.x, n.lo.y);
+            auto pnew = [&](uint32_t l, const FF2& z) {
+                P[l] = as4(ff2_add(z, ff2_mul(beta2, from4(P[l]))));
             };
-            // two slices (two ghosts) per step, their loads issued together
-            for (uint32_t s = s0 + warp; s < s1; s += 2 * nw) {
-                const uint32_t iA = s * 32 + lane, iB = iA + 32 * nw;
-                if (iA >= Nn) continue;
-                const bool vB = s + nw < s1 && iB < Nn;
-                const float4 rA = r4[iA];
-                const float2 dA = dinv[iA];
-                float4 rB{};
-                float2 dB{};
-                if (vB) {
-                    rB = r4[iB];
-                    dB = dinv[iB];
-                }
-                pnew(iA - s0 * 32, rA, dA);
-                if (vB) pnew(iB - s0 * 32, rB, dB);
-            }
+            // the ghosts from their owners' r, two per step, the loads issued
+            // together
             for (uint32_t j = tid; j < ng; j += 2 * kThreads) {
                 const uint32_t jB = j + kThreads;
                 const uint32_t cA = GID[j], cB = jB < ng ? GID[jB] : cA;
                 const float4 rA = r4[cA], rB = r4[cB];
                 const float2 dA = dinv[cA], dB = dinv[cB];
-                pnew(nslot + j, rA, dA);
-                if (jB < ng) pnew(nslot + jB, rB, dB);
+                pnew(nslot + j, ff2_mulf(from4(rA), dA));
+                if (jB < ng) pnew(nslot + jB, ff2_mulf(from4(rB), dB));
             }
+            // the own rows from z in shared memory
+            for (uint32_t l = tid; l < nslot && s0 * 32 + l < Nn; l += kThreads)
+                pnew(l, from4(W[l]));
             __syncthreads();
         }
     }
@@ -1132,7 +1139,7 @@ int ghost_setup(const nbg_bsr_t& A, unsigned G, char* plan, cudaStream_t s, Ghos
     uint32_t widest;
     if (!ghost_plan(A, G, plan, s, gh, &widest)) return 0;
     const size_t bytes = 16 * (size_t)gh->pcap + 16 * (size_t)gh->scap + 4 * (size_t)gh->gcap +
-                         (NBG_MIXED_SO_SMEM ? 4 * ((size_t)gh->scap / 32 + 1) : 0);
+                         4 * ((size_t)gh->scap / 32 + 1);
     if (!fits_smem((const void*)k_cg_mixed_ghost, kMixThreads, bytes, G)) return 0;
     *dyn = bytes;
     return 1;
