@@ -89,14 +89,6 @@ constexpr int kUnroll = NBG_MIXED_UNROLL;
 #ifndef NBG_BARRIER_COUNT
 #define NBG_BARRIER_COUNT 1
 #endif
-#ifndef NBG_L2_KEEP
-// percent of L2 for the matrix part kept between iterations (1M-dof ghost
-// form, us per iteration: 32.7 at 40, 31.3 at 35, 31.2 at 30, 32.7 at 25, 34.0
-// at 20: the rest of L2 holds the vectors); none for streams of over twice the
-// L2 (keep_permille)
-#define NBG_L2_KEEP 30
-#endif
-
 namespace {
 
 struct MixArgs {
@@ -111,15 +103,25 @@ struct MixArgs {
     double tol, delta;
     unsigned flags;
     int resident;      // own-row vectors live in shared memory
-    uint32_t keep_pm;  // per mille of each block's matrix stream kept in L2
+    uint32_t keep;     // share of each block's matrix stream kept in L2, of 2^32 (all ones: all)
 };
 
-// Whether the matrix of a block's slice `at` stays in L2 between iterations:
-// keep_pm / 1000 of the slices, spread evenly.  With the first ones kept,
-// DRAM had nothing to do while every warp worked on them (1M-dof ghost form:
-// 33.8 against 34.2 us per iteration).
-__device__ __forceinline__ bool kept(const MixArgs& a, uint32_t at) {
-    return (at + 1) * a.keep_pm / 1000u != at * a.keep_pm / 1000u;
+// Whether the matrix of slice `at` of a block's n stays in L2 between
+// iterations: a share `keep` of the slices.  With the first ones kept, DRAM had
+// nothing to do while every warp worked on them (1M-dof ghost form: 33.8
+// against 34.2 us per iteration); spread with a period, some pairs of warps,
+// which take every (kThreads / 64)th slice, had theirs all in L2 and others all
+// from DRAM (482,000 dof, half kept: 18.7 against 16.9).  So the fractional
+// parts of multiples of the golden ratio, along each pair's slices.  Batched
+// launches keep all or nothing (the test costs them 4 %).
+__device__ __forceinline__ bool kept_at(uint32_t j, uint32_t keep) {
+    return j * 0x9E3779B9u < keep || keep == 0xFFFFFFFFu;
+}
+template <int kThreads>
+__device__ __forceinline__ bool kept(const MixArgs& a, uint32_t at, uint32_t n) {
+    if (kThreads != kMixThreads) return a.keep != 0;
+    constexpr uint32_t kPairs = kThreads / 64;
+    return kept_at(at % kPairs * ((n + kPairs - 1) / kPairs) + at / kPairs, a.keep);
 }
 
 // One system of a launch: its slices, its blocks and its synchronisation.
@@ -490,7 +492,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
                 // a slice's rows past Nn are padding: skip them whole (both lanes)
                 if (s * 32 + ((h & 1) << 4) >= Nn) continue;
                 FF y0, y1;
-                const uint64_t pol = l2_policy(kept(a, s - s0));
+                const uint64_t pol = l2_policy(kept<kThreads>(a, s - s0, s1 - s0));
                 spmv_half_split(a, s, r, par, i < Nn, pol, y0, y1);
                 if (par || i >= Nn) continue;
                 o.w[li] = make_float4(y0.hi, y1.hi, y0.lo, y1.lo);
@@ -664,24 +666,31 @@ __global__ void __launch_bounds__(kBatThreads, kBatMinBlocks)
     mixed_solve<kOwn, kBatThreads>(a, sg, smem);
 }
 
-// Share of the SpMV's matrix stream (FP32 values, remainders, columns:
-// 32 B per block entry) marked evict_last: what fits in NBG_L2_KEEP percent
-// of this device's L2, the rest of L2 being left to the gathered vector and
-// the other data.
-uint32_t keep_permille(const nbg_bsr_t& A, double bytes_per_entry = 32.0) {
+// The SpMV's matrix stream (FP32 values, remainders, columns: 32 B per block
+// entry) in units of this device's L2; negative: not known.
+double stream_over_l2(const nbg_bsr_t& A, double bytes_per_entry = 32.0) {
     int dev = 0, l2 = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess)
-        return 0;
-    const double stream = bytes_per_entry * (double)A.n_entries;
-    const double budget = l2 * (NBG_L2_KEEP / 100.0);
-    // a stream of more than twice the L2 gains less from the kept part than
-    // its vectors lose (us per iteration without and with: q4 with 2.1M dof
-    // 80.0 and 86.4, T3 with 2.6M dof 99.4 and 106.6, at 1.6 times the L2
-    // 53.8 and 52.2)
-    if (stream > 2.0 * l2) return 0;
-    if (stream <= 0.0 || budget >= stream) return 1000;
-    return (uint32_t)(1000.0 * budget / stream);
+        cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess || l2 <= 0)
+        return -1.0;
+    return bytes_per_entry * (double)A.n_entries / l2;
+}
+
+// Share of the matrix stream marked evict_last (of 2^32): 45 % of L2 while the
+// stream and the vectors are not much larger than it, falling to 30 % from 1.4
+// times L2 on, where the rest of the stream pushes the vectors out.  Ghost
+// form, us per iteration with 30 % everywhere and with this rule (best of a
+// scan in steps of 50): 0.45 L2 14.7 and 14.4 (14.4), 0.57 18.1 and 17.3
+// (17.3), 0.63 19.0 and 17.8 (17.8), 0.69 21.1 and 20.7 (20.5), 0.87 25.1 and
+// 25.2 (25.1), 1.1 30.6 and 30.6 (30.6), 1.37 38.9 and 38.8 (38.5).  A stream of
+// more than twice the L2 gains less from the kept part than its vectors lose
+// (without and with: q4 with 2.1M dof 80.0 and 86.4, T3 with 2.6M dof 99.4 and
+// 106.6, at 1.6 times the L2 53.8 and 52.2).
+uint32_t keep_share(const nbg_bsr_t& A, double bytes_per_entry = 32.0) {
+    const double x = stream_over_l2(A, bytes_per_entry);
+    if (x <= 0.0 || x > 2.0) return 0;
+    const double share = std::min(0.45, std::max(0.30, 0.45 - (x - 0.7) * (0.15 / 0.7)));
+    return (uint32_t)(4294967295.0 * std::min(1.0, share / x));
 }
 
 // Vectors, partial sums, then what a launch needs at zero: barrier, status
@@ -709,7 +718,7 @@ size_t mixed_bytes(uint32_t N) { return mixed_core_bytes(N) + perm_tail_bytes(N)
 
 // The mixed solver's SpMV operator as its own launch: w = A p with the split
 // matrix and float-float p, two lanes per node row, the solver's L2 policy
-// (keep_pm / 1000 of each block's slices evict_last).  One block per
+// (a share `keep` of the slices evict_last).  One block per
 // SM, slices split evenly, as in the solver.
 __global__ void __launch_bounds__(kMixThreads, kMixMinBlocks)
     k_spmv_mixed(MixArgs a, float2* __restrict__ wh, float2* __restrict__ wl) {
@@ -722,7 +731,7 @@ __global__ void __launch_bounds__(kMixThreads, kMixMinBlocks)
         const uint32_t i = s * 32 + r;
         if (s * 32 + ((h & 1) << 4) >= a.A.Nn) continue;
         FF y0, y1;
-        const uint64_t pol = l2_policy(kept(a, s - s0));
+        const uint64_t pol = l2_policy(kept<kMixThreads>(a, s - s0, s1 - s0));
         spmv_half_split<true>(a, s, r, par, i < a.A.Nn, pol, y0, y1);
         if (par || i >= a.A.Nn) continue;
         wh[i] = make_float2(y0.hi, y1.hi);
@@ -922,7 +931,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
                 const uint32_t i = s * 32 + r, li = i - s0 * 32;
                 if (s * 32 + ((h & 1) << 4) >= Nn) continue;
                 FF y0, y1;
-                const uint64_t pol = l2_policy(kept(a, s - s0));
+                const uint64_t pol = l2_policy(kept<kThreads>(a, s - s0, s1 - s0));
                 spmv_half_local(a, gh.lcol, P, SO, s - s0, r, par, i < Nn, pol, y0, y1);
                 if (par || i >= Nn) continue;
                 W[li] = make_float4(y0.hi, y1.hi, y0.lo, y1.lo);
@@ -1107,7 +1116,7 @@ extern "C" int nbg_spmv_bsr_mixed(const nbg_bsr_t* A, const float* ph, const flo
     a.A = *A;
     a.ph = ph;
     a.pl = pl;
-    a.keep_pm = keep_permille(*A);
+    a.keep = keep_share(*A);
     unsigned G = 0;
     const int rc = coop_grid((const void*)k_spmv_mixed, A->n_slices, &G, kMixThreads);
     if (rc != NBG_OK) return rc;
@@ -1250,7 +1259,7 @@ extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint
     a.tol = tol;
     a.delta = delta;
     a.flags = flags;
-    a.keep_pm = keep_permille(*A);
+    a.keep = keep_share(*A);
     int rc = NBG_OK;
     unsigned G = 1;
     size_t dyn = 0;
@@ -1305,7 +1314,7 @@ extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint
     g.g_base = 0;
     g.g_size = G;
     g.pstride = kMaxBlocks;
-    if (ghost) a.keep_pm = keep_permille(*A, 30.0);
+    if (ghost) a.keep = keep_share(*A, 30.0);
     g_mixed_form = ghost ? NBG_MIXED_GHOST : slice_g || a.resident ? NBG_MIXED_RESIDENT_ROWS
                                                                   : NBG_MIXED_GLOBAL_ROWS;
     if (e == cudaSuccess && rc == NBG_OK) {
@@ -1499,7 +1508,8 @@ int batch_plan(nbg_mixed_batch* m, double gamma) {
     // all of a batch's matrix or nothing: a system reads its part again only
     // after every other system's (24 systems, 252 MB: 337 ms with none kept,
     // 351 with a fifth; 12 systems, 41 MB: 33.2 ms with all, 34.2 with none)
-    a.keep_pm = keep_permille(m->A) == 1000 ? 1000 : 0;
+    const double in_l2 = stream_over_l2(m->A);
+    a.keep = in_l2 > 0.0 && in_l2 <= 0.30 ? 0xFFFFFFFFu : 0;
     a.resident = own == 3;
     m->own = own;
     std::vector<Group> groups(n);

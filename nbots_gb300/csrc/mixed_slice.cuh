@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
     };
     uint64_t zepoch = 1;
-    const uint64_t pol = l2_policy(warp * 1000u < a.keep_pm * (s1 - s0));
+    const uint64_t pol = l2_policy(kept_at(warp, a.keep));
 
     // the resident entries of this warp's slice, then the others [e0, e1);
     // rows past Nn hold no entries
