@@ -340,14 +340,17 @@ int nbg_cg_mixed(const nbg_bsr_t *A, const double *b, double *x, uint32_t max_it
 /* Batched mixed-precision CG: n_sys independent systems stored as one
  * block-diagonal layout A, system i owning slices [slice_ptr[i],
  * slice_ptr[i+1]) (its node rows start on a multiple of 32), solved side by
- * side by one cooperative launch in which each system has its own group of
+ * side by cooperative launches in which each system has its own group of
  * blocks, barrier, reductions and stopping test.  A launch (x = 0, the
  * solve, then the optional SIMP compliance sensitivities with a = b = x) is
- * one CUDA graph replayed on `stream`.  Blocks are shared out in
- * proportion to slices^gamma (nbg_mixed_batch_plan, gamma 1.5 at creation);
- * nbg_mixed_batch_tune times one launch per candidate gamma and keeps the
- * fastest.  Every system needs a co-resident block: n_sys is at most the
- * launch's resident block count.  No counterpart in nbots. */
+ * one CUDA graph replayed on `stream`.  Systems of at most 28 slices per SM
+ * are solved in one or more waves with one block per SM and a warp for each
+ * slice, where that is faster; else all systems side by side.  Blocks are
+ * shared out in proportion to slices^gamma (nbg_mixed_batch_plan, gamma 1.5
+ * at creation); nbg_mixed_batch_tune times one launch per candidate gamma
+ * and keeps the fastest.  Every system needs a co-resident block: n_sys is at
+ * most the resident block count of the side-by-side launch.  No counterpart
+ * in nbots. */
 typedef struct nbg_mixed_batch nbg_mixed_batch_t;
 int nbg_mixed_batch_create(nbg_mixed_batch_t **out, const nbg_bsr_t *A, const double *b,
                            double *x, uint32_t n_sys, const uint32_t *slice_ptr,
@@ -355,7 +358,7 @@ int nbg_mixed_batch_create(nbg_mixed_batch_t **out, const nbg_bsr_t *A, const do
                            void *stream);
 void nbg_mixed_batch_destroy(nbg_mixed_batch_t *m);
 int nbg_mixed_batch_plan(nbg_mixed_batch_t *m, double gamma);
-/* Total blocks of the launch; blocks[i] per system and the gamma in use. */
+/* Total blocks of the launch or its waves; blocks[i] per system and the gamma in use. */
 uint32_t nbg_mixed_batch_blocks(const nbg_mixed_batch_t *m, uint32_t *blocks, double *gamma);
 int nbg_mixed_batch_set_sensitivity(nbg_mixed_batch_t *m, uint32_t nen, uint32_t N_elem,
                                     const double *nod, const uint32_t *conn, double nu,

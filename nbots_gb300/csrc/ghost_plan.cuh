@@ -31,10 +31,19 @@ struct GhostArgs {
 // memory) and the local column of each of its entries.  *fail is set when a
 // block has more outside references than kGhostKeys, more ghosts than
 // kGhostMax, or more than 65535 local columns; the solver then keeps the
-// global-gather form.
+// global-gather form.  A batched launch: block b has the slices from
+// pb.range[b].x to .y, belongs to system pb.system_of[b], whose own *fail is
+// pb.fail_stride ints further on for each, and fails too when its rows and
+// ghosts take more than pb.limit bytes at 16 per row and 36 per ghost.
+struct PlanBatch {
+    const uint2* range;
+    const uint32_t* system_of;
+    size_t limit;
+    uint32_t fail_stride;
+};
 __global__ void __launch_bounds__(1024, 1) k_ghost_plan(nbg_bsr_t A, uint16_t* lcol,
                                                       uint32_t* ids, uint32_t* count,
-                                                      int* fail) {
+                                                      int* fail, PlanBatch pb) {
     extern __shared__ __align__(16) uint32_t keys[];  // kGhostKeys
     __shared__ uint32_t s_n;
     __shared__ uint32_t s_scan[32];
@@ -43,6 +52,11 @@ __global__ void __launch_bounds__(1024, 1) k_ghost_plan(nbg_bsr_t A, uint16_t* l
     const uint32_t nw = bd >> 5;
     uint32_t s0, s1;
     slice_range(A.n_slices, s0, s1);
+    if (pb.range) {
+        s0 = pb.range[blockIdx.x].x;
+        s1 = pb.range[blockIdx.x].y;
+        fail += pb.system_of[blockIdx.x] * pb.fail_stride;
+    }
     const uint32_t n0 = s0 * 32, nslot = (s1 - s0) * 32;
     if (tid == 0) s_n = s_wide = 0;
     __syncthreads();
@@ -106,7 +120,8 @@ __global__ void __launch_bounds__(1024, 1) k_ghost_plan(nbg_bsr_t A, uint16_t* l
     }
     __syncthreads();
     const uint32_t u = s_scan[nw - 1];
-    if (u > kGhostMax || nslot + u > 65535u) {  // the same u in every thread
+    if (u > kGhostMax || nslot + u > 65535u ||
+        (pb.range && 16 * (size_t)nslot + 36 * (size_t)u + 16 > pb.limit)) {  // the same u in every thread
         if (tid == 0) atomicExch(fail, 1);
         return;
     }
@@ -155,15 +170,23 @@ size_t ghost_plan_bytes(const nbg_bsr_t& A) {
     return align256(2 * (size_t)A.n_entries) + align256(G * kGhostMax * 4) + align256(G * 8) + 256;
 }
 
+// Where the plan of a G-block partition stands in its workspace region.
+void ghost_regions(const nbg_bsr_t& A, unsigned G, char* plan, uint16_t** lcol, uint32_t** ids,
+                   uint32_t** count) {
+    *lcol = (uint16_t*)plan;
+    *ids = (uint32_t*)(plan + align256(2 * (size_t)A.n_entries));
+    *count = *ids + (size_t)G * kGhostMax;
+}
+
 // The ghost plan for a G-block partition of A and the sizes that its launch
 // needs: returns 1 and fills gh and *widest (entries of the longest slice
 // row), or 0 (the caller keeps a global-gather form).  plan: the
 // workspace region of ghost_plan_bytes(A).
 int ghost_plan(const nbg_bsr_t& A, unsigned G, char* plan, cudaStream_t s, GhostArgs* gh,
                uint32_t* widest) {
-    uint16_t* lcol = (uint16_t*)plan;
-    uint32_t* ids = (uint32_t*)(plan + align256(2 * (size_t)A.n_entries));
-    uint32_t* count = ids + (size_t)G * kGhostMax;
+    uint16_t* lcol;
+    uint32_t *ids, *count;
+    ghost_regions(A, G, plan, &lcol, &ids, &count);
     int* fail = (int*)((char*)count + align256((size_t)G * 8));
     int dev = 0, nsm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -175,7 +198,7 @@ int ghost_plan(const nbg_bsr_t& A, unsigned G, char* plan, cudaStream_t s, Ghost
                              (int)(kGhostKeys * 4)) != cudaSuccess)
         return 0;
     if (cudaMemsetAsync(fail, 0, sizeof(int), s) != cudaSuccess) return 0;
-    k_ghost_plan<<<G, 1024, kGhostKeys * 4, s>>>(A, lcol, ids, count, fail);
+    k_ghost_plan<<<G, 1024, kGhostKeys * 4, s>>>(A, lcol, ids, count, fail, PlanBatch{});
     if (cudaGetLastError() != cudaSuccess) return 0;
     std::vector<uint32_t> cnt(2 * (size_t)G);
     int hfail = 1;

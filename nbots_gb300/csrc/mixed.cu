@@ -1213,6 +1213,13 @@ const void* mixed_kernel(int own) {
                     : (const void*)k_cg_mixed<0>;
 }
 
+// slices per block of a batch's waves
+constexpr uint32_t kSlicesFew = 16, kSlicesMost = 28;
+const void* slices_kernel(int threads) {
+    return threads <= 32 * (int)kSlicesFew ? (const void*)k_cg_mixed_slices<32 * kSlicesFew>
+                                           : (const void*)k_cg_mixed_slices<32 * kSlicesMost>;
+}
+
 const void* batch_kernel(int own) {
     return own == 3 ? (const void*)k_cg_mixed_many<3>
          : own == 2 ? (const void*)k_cg_mixed_many<2>
@@ -1275,7 +1282,7 @@ extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint
     }
     GhostArgs gh;
     memset(&gh, 0, sizeof(gh));
-    SliceArgs sl{0, tail + 3 * 256};
+    SliceArgs sl{0, 0, (unsigned char*)tail + 3 * 256};
     bool ghost = false;
     int dev = 0, nsm = 0, threads = kMixThreads;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
@@ -1344,6 +1351,17 @@ extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint
 // cooperative launch of k_cg_mixed_many, replayed as a CUDA graph together
 // with zeroing x and, optionally, the SIMP compliance sensitivities.
 
+namespace {
+// One launch of the slice form (k_cg_mixed_slices): systems side by side, one
+// block per SM, a warp for each slice.
+struct Wave {
+    std::vector<uint32_t> systems, blocks;
+    uint32_t first;  // blocks of the waves before it
+    unsigned G;
+    int threads;
+};
+}  // namespace
+
 struct nbg_mixed_batch {
     nbg_bsr_t A;
     const double* b;
@@ -1362,7 +1380,11 @@ struct nbg_mixed_batch {
     unsigned char* d_state;
     unsigned G;
     size_t dyn;
-    int own;  // own-row vectors in shared memory (mixed_solve's kOwn)
+    int own;      // own-row vectors in shared memory (mixed_solve's kOwn), or kSliceForm
+    std::vector<Wave> waves;  // slice form: its launches, one after the other
+    unsigned char* d_sums;    // kBatchSums per system
+    uint2* d_range;           // slices of each block
+    char* d_plan;             // ghost plan; null: not for the slice form
     // compliance sensitivities after the solve (a = b = x)
     bool sens;
     uint32_t nen, N_elem;
@@ -1377,7 +1399,9 @@ struct nbg_mixed_batch {
 
 namespace {
 
-constexpr size_t kStateStride = 256;  // per system: barrier at +0, status at +128
+constexpr size_t kStateStride = 256;  // per system: barrier +0, status +128, plan failed +192
+constexpr size_t kBatchSums = kArBytes + 2 * kExactBytes;  // per system, of the slice form
+constexpr int kSliceForm = 4;  // nbg_mixed_batch::own
 constexpr size_t kResStride = 8;      // doubles of result per system
 
 size_t batch_bytes(uint32_t N, uint32_t n_sys) {
@@ -1395,22 +1419,25 @@ double* part_slots(char* base, uint32_t N) {
     return (double*)(base + 6 * f + 2 * h);
 }
 
-// Blocks per system: one each, then one at a time to the system with the
-// largest weight per block (weight = slices^gamma), never more blocks than
-// warps of slices.  Minimises the largest weight per block.
+// Blocks per system: one each (or enough for most_per_block slices), then one
+// at a time to the system with the largest weight per block (weight =
+// slices^gamma), never more than one per least_per_block slices.  Minimises
+// the largest weight per block.
 void share_blocks(const std::vector<uint32_t>& sp, double gamma, unsigned total,
-                  std::vector<uint32_t>& out) {
+                  uint32_t least_per_block, uint32_t most_per_block, std::vector<uint32_t>& out) {
     const size_t n = sp.size() - 1;
-    const uint32_t nw = kBatThreads / 32;
     std::vector<double> w(n);
     std::vector<uint32_t> cap(n);
     out.assign(n, 1);
+    unsigned used = 0;
     for (size_t i = 0; i < n; i++) {
         const uint32_t S = sp[i + 1] - sp[i];
         w[i] = std::pow((double)std::max<uint32_t>(S, 1), gamma);
-        cap[i] = std::max<uint32_t>(1, (S + nw - 1) / nw);
+        cap[i] = std::max<uint32_t>(1, (S + least_per_block - 1) / least_per_block);
+        if (most_per_block) out[i] = std::max<uint32_t>(1, (S + most_per_block - 1) / most_per_block);
+        used += out[i];
     }
-    for (unsigned left = total - (unsigned)n; left > 0; --left) {
+    for (unsigned left = total - used; left > 0; --left) {
         size_t best = n;
         double bw = -1.0;
         for (size_t i = 0; i < n; i++)
@@ -1428,6 +1455,74 @@ uint32_t max_slices_per_block(const std::vector<uint32_t>& sp, const std::vector
     for (size_t i = 0; i + 1 < sp.size(); i++)
         m = std::max(m, (sp[i + 1] - sp[i] + bl[i] - 1) / bl[i]);
     return m;
+}
+
+// The systems in waves of at most `most` slices per block, as few as first-fit
+// decreasing finds; the time that they take, in us per square root of slices (an
+// iteration's time, and iterations grow with a mesh's length), or a negative
+// number when a system is too large.  Measured us per iteration of a wave: 4.5
+// with 4 slices per block, 5.6 with 16, the most that leaves a thread 128
+// registers, 7.0 with 17, 8.9 with 27, 11.6 with 32 (which is not used).
+double slice_waves(const std::vector<uint32_t>& sp, double gamma, unsigned total, uint32_t most,
+                   std::vector<Wave>& waves) {
+    const uint32_t n = (uint32_t)sp.size() - 1;
+    auto slices = [&](uint32_t i) { return sp[i + 1] - sp[i]; };
+    auto least = [&](uint32_t i) { return std::max(1u, (slices(i) + most - 1) / most); };
+    std::vector<uint32_t> order(n);
+    for (uint32_t i = 0; i < n; i++) order[i] = i;
+    std::stable_sort(order.begin(), order.end(),
+                     [&](uint32_t i, uint32_t j) { return slices(i) > slices(j); });
+    waves.clear();
+    if (least(order[0]) > total) return -1.0;
+    for (uint32_t i : order) {
+        auto w = std::find_if(waves.begin(), waves.end(),
+                              [&](const Wave& v) { return v.G + least(i) <= total; });
+        if (w == waves.end()) w = waves.insert(waves.end(), Wave{{}, {}, 0, 0, 0});
+        w->systems.push_back(i);
+        w->G += least(i);
+    }
+    double cost = 0.0;
+    uint32_t first = 0;
+    for (Wave& w : waves) {
+        std::vector<uint32_t> own{0};
+        for (uint32_t i : w.systems) own.push_back(own.back() + slices(i));
+        share_blocks(own, gamma, total, kSlicesFew, most, w.blocks);
+        const uint32_t per = std::max(1u, max_slices_per_block(own, w.blocks));
+        w.threads = 32 * (int)per;
+        w.first = first;
+        w.G = 0;
+        for (uint32_t v : w.blocks) w.G += v;
+        first += w.G;
+        cost += std::sqrt((double)slices(w.systems[0])) *
+                (per <= kSlicesFew ? 4.2 + 0.085 * per : 7.0 + 0.18 * (per - kSlicesFew - 1));
+    }
+    return first <= kMaxBlocks ? cost : -1.0;
+}
+
+// The better of two packings, when it beats all systems side by side in the
+// other form, whose iteration takes 8 us and 1.7 ns per slice: that is bound by
+// DRAM once the systems are larger than L2, while a wave's matrices are in shared
+// memory and L2; but a wave's block works for one system, however small.
+// Milliseconds in the other form and in waves: 24 systems of 48 and 96
+// elements' length 12.5 and 7.0, 6 of 96 and 192 25.0 and 11.1, 12 of 64 to 256
+// 50.0 and 30.3, 24 of 48 to 192 40.0 and 33.6, 24 of 64 to 512 277 and 259; 20 of
+// 96 to 384, six of them of 2,323 slices, stay (180, in waves 196).
+bool best_waves(const std::vector<uint32_t>& sp, double gamma, unsigned nsm,
+                std::vector<Wave>& waves) {
+    uint32_t largest = 0;
+    for (size_t i = 0; i + 1 < sp.size(); i++) largest = std::max(largest, sp[i + 1] - sp[i]);
+    double best = std::sqrt((double)largest) * (8.0 + 0.0017 * sp.back());
+    waves.clear();
+    for (uint32_t most : {kSlicesFew, kSlicesMost}) {
+        std::vector<Wave> w;
+        const double cost =
+            NBG_MIXED_RESIDENT ? slice_waves(sp, gamma, std::min(nsm, kExactMaxBlocks), most, w) : -1.0;
+        if (cost >= 0.0 && cost < best) {
+            best = cost;
+            waves.swap(w);
+        }
+    }
+    return !waves.empty();
 }
 
 inline int cu(cudaError_t e) { return e == cudaSuccess ? NBG_OK : nbg_cuda_error(e); }
@@ -1457,7 +1552,7 @@ int batch_plan(nbg_mixed_batch* m, double gamma) {
         NBG_CHECK(allow_smem(fn, &most));
         const unsigned total = std::min<unsigned>((unsigned)nsm * per_sm, kMaxBlocks);
         if (n > total) return NBG_OK;
-        share_blocks(m->slice_ptr, gamma, total, bl);
+        share_blocks(m->slice_ptr, gamma, total, kBatThreads / 32, 0, bl);
         const size_t bytes =
             (size_t)max_slices_per_block(m->slice_ptr, bl) * own_node_bytes(own) * 32;
         if (bytes > most) return NBG_OK;
@@ -1471,6 +1566,29 @@ int batch_plan(nbg_mixed_batch* m, double gamma) {
         }
         return NBG_OK;
     };
+    // the resident block count of the form that takes any systems
+    int occ0 = 0;
+    NBG_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ0, batch_kernel(0), kBatThreads, 0));
+    const unsigned total0 = std::min<unsigned>((unsigned)nsm * (unsigned)std::max(occ0, 1), kMaxBlocks);
+    if (n > total0) return NBG_ERR_ARG;  // every system needs a co-resident block
+    // the slice form where it takes the systems
+    std::vector<Wave> waves;
+    if (m->d_plan && best_waves(m->slice_ptr, gamma, (unsigned)nsm, waves)) {
+        NBG_CHECK(cudaFuncSetAttribute((const void*)k_ghost_plan,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(kGhostKeys * 4)));
+        own = kSliceForm;
+        bl.assign(n, 0);
+        for (const Wave& w : waves) {
+            size_t most = 0;
+            NBG_CHECK(allow_smem(slices_kernel(w.threads), &most));
+            dyn = dyn ? std::min(dyn, most) : most;
+            G += w.G;
+            for (size_t k = 0; k < w.systems.size(); k++) bl[w.systems[k]] = w.blocks[k];
+        }
+    } else {
+        waves.clear();
+    }
     // all own rows in shared memory, with fewer blocks per SM if need be;
     // else at the full block count as many of the vectors as fit
     for (int per_sm = kBatMinBlocks; own == 3 && per_sm >= 1 && !G; --per_sm) {
@@ -1484,12 +1602,7 @@ int batch_plan(nbg_mixed_batch* m, double gamma) {
     }
     if (!G) {
         own = 0;
-        const void* fn = batch_kernel(0);
-        int occ = 0;
-        NBG_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kBatThreads, 0));
-        const unsigned total = std::min<unsigned>((unsigned)nsm * (unsigned)std::max(occ, 1), kMaxBlocks);
-        if (n > total) return NBG_ERR_ARG;  // every system needs a co-resident block
-        share_blocks(m->slice_ptr, gamma, total, bl);
+        share_blocks(m->slice_ptr, gamma, total0, kBatThreads / 32, 0, bl);
         for (uint32_t v : bl) G += v;
         dyn = 0;
     }
@@ -1509,8 +1622,8 @@ int batch_plan(nbg_mixed_batch* m, double gamma) {
     // after every other system's (24 systems, 252 MB: 337 ms with none kept,
     // 351 with a fifth; 12 systems, 41 MB: 33.2 ms with all, 34.2 with none)
     const double in_l2 = stream_over_l2(m->A);
-    a.keep = in_l2 > 0.0 && in_l2 <= 0.30 ? 0xFFFFFFFFu : 0;
-    a.resident = own == 3;
+    a.keep = own == kSliceForm || (in_l2 > 0.0 && in_l2 <= 0.30) ? 0xFFFFFFFFu : 0;
+    a.resident = own >= 3;
     m->own = own;
     std::vector<Group> groups(n);
     std::vector<uint32_t> map(G);
@@ -1523,7 +1636,7 @@ int batch_plan(nbg_mixed_batch* m, double gamma) {
         g.bar = (unsigned*)(m->d_state + i * kStateStride);
         g.status = (int*)(m->d_state + i * kStateStride + 128);
         g.res = m->d_res + i * kResStride;
-        g.sums = nullptr;
+        g.sums = own == kSliceForm ? m->d_sums + i * kBatchSums + kArBytes : nullptr;
         g.s_begin = m->slice_ptr[i];
         g.s_end = m->slice_ptr[i + 1];
         g.g_base = gb;
@@ -1531,8 +1644,25 @@ int batch_plan(nbg_mixed_batch* m, double gamma) {
         for (uint32_t k = 0; k < bl[i]; k++) map[gb + k] = i;
         gb += bl[i];
     }
+    std::vector<uint2> range(G);
+    for (const Wave& w : waves) {  // blocks numbered within their wave
+        uint32_t at = 0;
+        for (uint32_t i : w.systems) {
+            const uint64_t S = m->slice_ptr[i + 1] - m->slice_ptr[i];
+            groups[i].g_base = at;
+            for (uint32_t k = 0; k < bl[i]; k++) {  // as group_slice_range
+                map[w.first + at + k] = i;
+                range[w.first + at + k] = make_uint2(m->slice_ptr[i] + (uint32_t)(S * k / bl[i]),
+                                                     m->slice_ptr[i] + (uint32_t)(S * (k + 1) / bl[i]));
+            }
+            at += bl[i];
+        }
+    }
     NBG_CHECK(cudaMemcpy(m->d_groups, groups.data(), n * sizeof(Group), cudaMemcpyHostToDevice));
     NBG_CHECK(cudaMemcpy(m->d_map, map.data(), G * 4, cudaMemcpyHostToDevice));
+    if (own == kSliceForm)
+        NBG_CHECK(cudaMemcpy(m->d_range, range.data(), G * sizeof(uint2), cudaMemcpyHostToDevice));
+    m->waves = waves;
     m->blocks = bl;
     m->G = G;
     m->dyn = dyn;
@@ -1546,9 +1676,10 @@ cudaError_t batch_enqueue(nbg_mixed_batch* m, cudaStream_t s) {
     cudaError_t e = cudaMemsetAsync(m->x, 0, 8 * (size_t)m->A.N, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(m->d_state, 0, (size_t)m->n_sys * kStateStride, s);
     if (e != cudaSuccess) return e;
+    const Group* groups = m->d_groups;
+    const uint32_t* map = m->d_map;
+    MixArgs args = m->args;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(m->G);
-    cfg.blockDim = dim3(kBatThreads);
     cfg.dynamicSmemBytes = m->dyn;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -1556,11 +1687,37 @@ cudaError_t batch_enqueue(nbg_mixed_batch* m, cudaStream_t s) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const Group* groups = m->d_groups;
-    const uint32_t* map = m->d_map;
-    MixArgs args = m->args;
-    void* params[] = {&args, &groups, &map};
-    e = cudaLaunchKernelExC(&cfg, batch_kernel(m->own), params);
+    if (m->own != kSliceForm) {
+        cfg.gridDim = dim3(m->G);
+        cfg.blockDim = dim3(kBatThreads);
+        void* params[] = {&args, &groups, &map};
+        e = cudaLaunchKernelExC(&cfg, batch_kernel(m->own), params);
+    } else {
+        e = cudaMemsetAsync(m->d_sums, 0, (size_t)m->n_sys * kBatchSums, s);
+    }
+    for (const Wave& w : m->waves) {
+        if (e != cudaSuccess) return e;
+        // planned in each launch, from the columns that the layout has then
+        GhostArgs gh;
+        memset(&gh, 0, sizeof(gh));
+        uint16_t* lcol;
+        uint32_t *ids, *count;
+        ghost_regions(m->A, w.G, m->d_plan, &lcol, &ids, &count);
+        gh.lcol = lcol;
+        gh.ids = ids;
+        gh.count = count;
+        map = m->d_map + w.first;
+        const PlanBatch pb{m->d_range + w.first, map, m->dyn, (uint32_t)(kStateStride / 4)};
+        k_ghost_plan<<<w.G, 1024, kGhostKeys * 4, s>>>(
+            m->A, lcol, ids, count, (int*)(m->d_state + 128) + kNoPlan, pb);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        SliceArgs sl{0, (uint32_t)m->dyn, nullptr};
+        cfg.gridDim = dim3(w.G);
+        cfg.blockDim = dim3(w.threads);
+        void* params[] = {&args, &groups, &map, &gh, &sl};
+        e = cudaLaunchKernelExC(&cfg, slices_kernel(w.threads), params);
+    }
     if (e != cudaSuccess || !m->sens) return e;
     const int rc = nbg_simp_sensitivity_f64(m->nen, m->N_elem, m->nod, m->conn, m->nu,
                                             m->thickness, m->rho, m->penal, m->E0, m->Emin, m->x,
@@ -1618,8 +1775,15 @@ extern "C" int nbg_mixed_batch_create(nbg_mixed_batch_t** out, const nbg_bsr_t* 
     m->delta = delta;
     m->flags = flags;
     m->stream = (cudaStream_t)stream;
-    const size_t need = batch_bytes(A->N, n_sys);
-    cudaError_t e = cudaMalloc(&m->ws, need);
+    std::vector<Wave> waves;
+    int dev = 0, nsm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const bool slices = e == cudaSuccess && best_waves(m->slice_ptr, 1.5, (unsigned)nsm, waves);
+    const size_t base_bytes = batch_bytes(A->N, n_sys), sums = align256((size_t)n_sys * kBatchSums),
+                 ranges = align256(sizeof(uint2) * kMaxBlocks);
+    const size_t need = base_bytes + (slices ? sums + ranges + ghost_plan_bytes(*A) : 0);
+    if (e == cudaSuccess) e = cudaMalloc(&m->ws, need);
     if (e != cudaSuccess) {
         delete m;
         return nbg_cuda_error(e);
@@ -1632,6 +1796,10 @@ extern "C" int nbg_mixed_batch_create(nbg_mixed_batch_t** out, const nbg_bsr_t* 
     m->d_groups = (Group*)p;
     p += align256((size_t)n_sys * sizeof(Group));
     m->d_map = (uint32_t*)p;
+    p = (char*)m->ws + base_bytes;
+    m->d_sums = (unsigned char*)p;
+    m->d_range = (uint2*)(p + sums);
+    m->d_plan = slices ? p + sums + ranges : nullptr;
     // weights slices^1.5: CG's iterations grow with a mesh's length, so with
     // shares in proportion to the slices the small systems finish early and
     // their blocks idle (24 systems of 64 to 512 elements' length: 377 ms at

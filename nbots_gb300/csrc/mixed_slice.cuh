@@ -32,8 +32,11 @@
 // the same bits.
 
 struct SliceArgs {
-    uint32_t keep;     // entries of each row in shared memory
-    void* ar;          // the sums' records (kArBytes) and words (2 kExactBytes), zero at launch
+    uint32_t keep;  // entries of each row in shared memory (batched: as many as fit)
+    uint32_t dyn;   // bytes of dynamic shared memory
+    // the sums' records (kArBytes) and words (2 kExactBytes), zero at launch
+    // (batched: the group's)
+    unsigned char* ar;
 };
 
 // The resident entries of one row, those of the k-th column at [k * 32]
@@ -109,10 +112,10 @@ __device__ __forceinline__ void publish_z(unsigned char* zx, unsigned char* zy, 
 }
 
 // kThreads: the largest block; 512 threads leave 128 registers each.
-template <bool kGhost, int kThreads>
-__global__ void __launch_bounds__(kThreads, 1)
-    k_cg_mixed_slice(MixArgs a, Group g, GhostArgs gh, SliceArgs sl) {
-    extern __shared__ __align__(16) unsigned char smem[];
+// kBatch: one of several systems in the launch.
+template <bool kGhost, bool kBatch, int kThreads>
+__device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, const GhostArgs& gh,
+                                            const SliceArgs& sl, unsigned char* smem) {
     __shared__ double red[3 * 32];
     __shared__ int s_sum1[kSumShared], s_sum2[kSumShared];
     __shared__ uint64_t s_ff[2 * 32];
@@ -122,22 +125,28 @@ __global__ void __launch_bounds__(kThreads, 1)
     __shared__ int s_fail;   // a wait for ghosts or records ran out
     __shared__ int s_again;  // the fixed-point sum's status: 1 sum by records, 2 give up
     __shared__ MixScalars sc;  // thread 0 only
-    const unsigned G = gridDim.x;
-    const uint32_t rank = blockIdx.x;
+    const unsigned G = kBatch ? g.g_size : gridDim.x;
+    const uint32_t rank = kBatch ? blockIdx.x - g.g_base : blockIdx.x;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t bd = blockDim.x, nw = bd >> 5;
     uint32_t s0, s1;
-    slice_range(a.A.n_slices, s0, s1);
+    if (kBatch) group_slice_range(g.s_begin, g.s_end, rank, G, s0, s1);
+    else slice_range(a.A.n_slices, s0, s1);
     const uint32_t Nn = a.A.Nn, nslot = (s1 - s0) * 32;
     const uint32_t s = s0 + warp, i = s * 32 + lane, li = warp * 32 + lane;
     const bool live = warp < s1 - s0 && i < Nn;
-    const uint32_t ng = kGhost ? gh.count[rank] : 0;
+    const uint32_t ng = kGhost ? gh.count[blockIdx.x] : 0;
+    const uint32_t pcap = kBatch ? nslot + ng : gh.pcap, gcap = kBatch ? ng : gh.gcap;
     // shared memory: p of rows and ghosts, z of the ghosts, ghost ids, matrix
     float4* const P = reinterpret_cast<float4*>(smem);
-    float4* const ZG = P + gh.pcap;
-    uint32_t* const GID = reinterpret_cast<uint32_t*>(ZG + gh.gcap);
-    float4* const mat = reinterpret_cast<float4*>(GID + ((gh.gcap + 3) & ~3u));
-    const uint32_t cap = nw * sl.keep * 32, m0 = warp * sl.keep * 32 + lane;
+    float4* const ZG = P + pcap;
+    uint32_t* const GID = reinterpret_cast<uint32_t*>(ZG + gcap);
+    float4* const mat = reinterpret_cast<float4*>(GID + ((gcap + 3) & ~3u));
+    const uint32_t keep =
+        kBatch && kGhost ? (uint32_t)((sl.dyn - ((unsigned char*)mat - smem)) /
+                                      (slice_entry_bytes(kThreads) * bd))
+                         : sl.keep;
+    const uint32_t cap = nw * keep * 32, m0 = warp * keep * 32 + lane;
     constexpr bool kDecoded = slice_decoded(kThreads);
     uint32_t* const mat2 = reinterpret_cast<uint32_t*>(mat + cap);
     const SliceMatrix sm = {mat + m0, mat + cap + m0, reinterpret_cast<const uint2*>(mat2) + m0,
@@ -150,6 +159,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     double* const part2 = g.part + 3 * g.pstride;
     double2* __restrict__ u = reinterpret_cast<double2*>(a.u);
     const double2* __restrict__ b = reinterpret_cast<const double2*>(a.b);
+    auto area = [&]() { return kBatch ? g.sums - kArBytes : sl.ar; };
     unsigned bar_target = 0;
     auto sync = [&]() { return grid_barrier_count(g.bar, G, bar_target, g.status); };
     __shared__ ExactSum sum1, sum2;  // p.w; r.z and |r|^2
@@ -158,7 +168,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     auto by_records = [&](auto& v) {
         constexpr int kNV = sizeof(v) / sizeof(FF);
         AllReduce ar;
-        ar.init(sl.ar, g.status, G, rank);
+        ar.init(area(), g.status, G, rank);
         ar.epoch = s_epoch;
         block_sum_end<SumFF, kNV>(v, s_ff, nw);
         const int fail = ar.sum<SumFF, kNV>(v);
@@ -175,7 +185,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint32_t e0 = 0, e1 = 0, n_res = 0;
     if (live) {
         const uint32_t k0 = a.A.slice_off[s], k1 = a.A.slice_off[s + 1];
-        n_res = kGhost ? min(k1 - k0, sl.keep) : 0;
+        n_res = kGhost ? min(k1 - k0, keep) : 0;
         for (uint32_t k = 0; k < n_res; k++) {
             const uint32_t e = (k0 + k) * 32 + lane;
             const_cast<float4*>(sm.hi)[k * 32] = reinterpret_cast<const float4*>(a.A.b32)[e];
@@ -249,11 +259,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         sc.clear();
         s_fail = 0;
         s_epoch = 0;
-        sum1.init((unsigned char*)sl.ar + kArBytes);
-        sum2.init((unsigned char*)sl.ar + kArBytes + kExactBytes);
+        sum1.init(area() + kArBytes);
+        sum2.init(area() + kArBytes + kExactBytes);
     }
     if (kGhost) {
-        for (uint32_t j = tid; j < ng; j += bd) GID[j] = gh.ids[(size_t)rank * kGhostMax + j];
+        for (uint32_t j = tid; j < ng; j += bd) GID[j] = gh.ids[(size_t)blockIdx.x * kGhostMax + j];
         // no record of an earlier solve may look current
         if (live) {
             st_record(zx + (size_t)i * 16, 0, 0);
@@ -477,4 +487,26 @@ done:
         g.res[3] = sc.rr64;
         g.res[4] = sc.bb;
     }
+}
+
+template <bool kGhost, int kThreads>
+__global__ void __launch_bounds__(kThreads, 1)
+    k_cg_mixed_slice(MixArgs a, Group g, GhostArgs gh, SliceArgs sl) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    slice_solve<kGhost, false, kThreads>(a, g, gh, sl, smem);
+}
+
+// Batched: block b works for system groups[block_of[b]], with its ghosts where
+// the plan found room for them in all of the system's blocks.
+constexpr int kNoPlan = 16;  // ints from a system's status to its plan's failure flag
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 1)
+    k_cg_mixed_slices(MixArgs a, const Group* __restrict__ groups,
+                      const uint32_t* __restrict__ block_of, GhostArgs gh, SliceArgs sl) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ Group sg;
+    if (threadIdx.x == 0) sg = groups[block_of[blockIdx.x]];
+    __syncthreads();
+    if (sg.status[kNoPlan] == 0) slice_solve<true, true, kThreads>(a, sg, gh, sl, smem);
+    else slice_solve<false, true, kThreads>(a, sg, gh, sl, smem);
 }
