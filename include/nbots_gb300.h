@@ -183,6 +183,10 @@ int nbg_spmv_csr_f64(uint32_t N, const uint32_t *row_ptr, const uint32_t *col_id
  * lagged ||g|| of the previous iteration, reported as tol_reached (else the
  * current ||g||, confirmed on the true residual b - A x) */
 #define NBG_CG_NBOTS_STOP 4u
+/* nbg_cg_bsr_f64: one order of summation, whatever the workspace holds (the
+ * global form).  Two orders stop an iteration apart now and then, which what is
+ * derived from the solution (strains) shows. */
+#define NBG_CG_FIXED_ORDER 8u
 
 typedef struct {
     uint32_t niter;       /* iterations performed */

@@ -200,7 +200,8 @@ int nbg_fem_damage(nbg_fem_t *f, const nbg_bcs_t *bcs, double E, double nu, doub
 				TRY(nbg_fem_block_layout(f, NULL));  /* from this K */
 				st = nbg_cg_bsr_f64(&f->bsr, w.res, w.du, N, 1e-8,
 						    method == NBG_METHOD_NBOTS_FAST
-							    ? NBG_CG_JACOBI | NBG_CG_NBOTS_STOP
+							    ? NBG_CG_JACOBI | NBG_CG_NBOTS_STOP |
+							      NBG_CG_FIXED_ORDER
 							    : NBG_CG_JACOBI,
 						    &cg, w.bws, bws_bytes, f->stream);
 			} else {

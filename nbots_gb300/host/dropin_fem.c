@@ -241,7 +241,8 @@ int nb_fem_compute_2D_Solid_Mechanics(const nb_mesh2D_t *part, const nb_fem_elem
 		nbg_cg_result_t r;
 		int st = exact_cg() ? nbg_fem_solve(f, nbg_fem_n_dof(f), 1e-8, NBG_CG_JACOBI, &r)
 				    : nbg_fem_solve_fast(f, nbg_fem_n_dof(f), 1e-8,
-							 NBG_CG_JACOBI | NBG_CG_NBOTS_STOP, &r);
+							 NBG_CG_JACOBI | NBG_CG_NBOTS_STOP |
+								 NBG_CG_FIXED_ORDER, &r);
 		rc = st < 0 ? st : NBG_OK;
 	}
 	if (rc == NBG_OK)
