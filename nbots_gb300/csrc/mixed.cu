@@ -27,7 +27,8 @@
 // `delta` since the last one; p is kept, so the Krylov progress survives.
 // Convergence is judged on the FP64 residual only.  Three grid barriers per
 // iteration in the global-gather form (L1 | L2 | L3 of
-// cg_precond_jacobi.c:50-74), two in the ghost-node form below: folding L3
+// cg_precond_jacobi.c:50-74), two sums over the grid in the ghost-node form
+// below and in the slice form (mixed_slice.cuh): folding L3
 // into the next SpMV (each block rebuilding z + beta p for the columns it
 // reads) measured slower, 77 vs 66 us per iteration at 1M dof, because the
 // float-float rebuild per column costs more issue slots and gather bytes
@@ -282,6 +283,11 @@ struct Own {
     float4 *p, *x, *r, *w;  // {hi, hi, lo, lo}
     const float2* dv;
 };
+// Up to 192 KB per SM for them: the L1 cache left beside more holds too few of
+// the SpMV's gathers (us per iteration with nothing, A p, and A p and r in shared
+// memory: T3 of 1.28M nodes 99.0, 92.8 at 135 KB; 1.8M 146.9, 135.3 at 190 KB; 2.0M
+// 163.2, 191.3 at 211 KB; Q4 of 1.02M 78.1, 75.3, 89.1 at 215 KB).
+constexpr size_t kOwnSmem = 192 * 1024;
 constexpr size_t own_node_bytes(int own) { return own == 3 ? 64 : 16 * (size_t)own; }
 
 template <int kOwn>
@@ -1313,7 +1319,7 @@ extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint
             rc = coop_grid_resident(fn, A->n_slices, own_node_bytes(own) * 32, &G, &dyn, kMixThreads,
                                     kMixMinBlocks);
             a.resident = own == 3;
-            if (own > 0 && dyn == 0) fn = nullptr;
+            if (own > 0 && (dyn == 0 || (own < 3 && dyn > kOwnSmem))) fn = nullptr;
         }
     }
     g.s_begin = 0;
@@ -1555,7 +1561,7 @@ int batch_plan(nbg_mixed_batch* m, double gamma) {
         share_blocks(m->slice_ptr, gamma, total, kBatThreads / 32, 0, bl);
         const size_t bytes =
             (size_t)max_slices_per_block(m->slice_ptr, bl) * own_node_bytes(own) * 32;
-        if (bytes > most) return NBG_OK;
+        if (bytes > most || (own < 3 && bytes * per_sm > kOwnSmem)) return NBG_OK;
         int occ = 0;
         NBG_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kBatThreads, bytes));
         unsigned used = 0;

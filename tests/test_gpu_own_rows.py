@@ -15,10 +15,10 @@ pytestmark = pytest.mark.gpu
 BUDGET, RTOL = 40, 1e-8
 
 
-# node rows per SM: 110 and 112 slices of 32, 225 and 228, 451 and 454
-# (2 KiB per slice for all vectors, 1 KiB, 512 B, of 227 KiB per SM)
-@pytest.mark.parametrize("nx,ny", [(799, 667), (799, 681), (1023, 1068), (1023, 1083),
-                                   (1999, 1097), (1999, 1105)])
+# slices of 32 node rows per SM: 110 and 113 (2 KiB each for all vectors, of
+# 227 KiB), 192 and 193, 384 and 386 (1 KiB for two, 512 B for one, of 192 KiB)
+@pytest.mark.parametrize("nx,ny", [(799, 667), (799, 681), (1023, 911), (1023, 914),
+                                   (1999, 932), (1999, 936)])
 def test_single_system(nx, ny):
     from nbots_gb300 import _lib as L, workloads as W
     from nbots_gb300.device import DeviceArray
@@ -43,8 +43,9 @@ def test_single_system(nx, ny):
 
 
 # 3,738 slices per system: 98 per SM (all vectors), 123 (31 per block: two),
-# 221 (56 per block: one), 443 (111 per block: none)
-@pytest.mark.parametrize("count", [4, 5, 9, 18])
+# 221 (56 per block: one), 443 (111 per block: none); at 7, 172 (43 per block: two)
+# and at 8, 197 (50 per block: one)
+@pytest.mark.parametrize("count", [4, 5, 7, 8, 9, 18])
 def test_batch(count):
     from nbots_gb300 import _lib as L, workloads as W
     from nbots_gb300.batch import Batch
