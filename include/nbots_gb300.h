@@ -323,13 +323,15 @@ int nbg_spmv_bsr_mixed(const nbg_bsr_t *A, const float *ph, const float *pl, flo
 
 /* Workspace: nbg_cg_mixed_workspace_bytes(N) at least.  With
  * nbg_cg_mixed_layout_workspace_bytes(A) (more: a 16-bit local column per
- * layout entry and per-block ghost lists) the solver takes its ghost-node
+ * layout entry and per-block ghost lists) the solver takes a ghost-node
  * form when the system is small enough for each block's rows and ghosts to
  * live in shared memory: every block keeps the search direction p of its
- * own rows and of the rows its rows couple to (its ghosts) on chip, updates
- * the ghosts itself from their owners' published residual, and so needs
- * two grid barriers per iteration instead of three; the iterates are the
- * same bit for bit.  ws NULL allocates the larger size. */
+ * own rows and of the rows its rows couple to (its ghosts) on chip and
+ * updates the ghosts itself from what their owners publish, so that an
+ * iteration has two sums over the grid and no exchange of p; the iterates
+ * are the same bit for bit.  Up to 32 slices per SM (311,000 dof) a warp owns
+ * a slice (the slice form, with or without ghosts).  ws NULL allocates the
+ * larger size. */
 size_t nbg_cg_mixed_workspace_bytes(uint32_t N);
 size_t nbg_cg_mixed_layout_workspace_bytes(const nbg_bsr_t *A);
 /* The form the calling thread's last nbg_cg_mixed launch took. */

@@ -1,6 +1,8 @@
 // Fast persistent FP64 (Jacobi-preconditioned) CG on the 2x2-block SELL
-// layout (bsr.cu): one cooperative launch per solve, one thread per node
-// row, convergence decided on the device, every spin bounded.
+// layout (bsr.cu): one cooperative launch per solve, convergence decided on
+// the device, every spin bounded.  Two forms: the slice form
+// (cg_bsr_slice.cuh) up to 32 slices per SM when the workspace holds its
+// plan, and the global form here, one thread per node row.
 //
 // GB300 issues FP64 at a small fraction of its FP32 rate, so this kernel
 // keeps the FP64 instruction count at one FMA per stored value plus seven
