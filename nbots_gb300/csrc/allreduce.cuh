@@ -223,6 +223,19 @@ constexpr int kSumWords = kLimbs + 1;  // per value: the limbs, values outside t
 // line of its own; zero at launch
 constexpr size_t kExactBytes = 2 * 128;
 constexpr unsigned kExactMaxBlocks = 255;  // counted in a byte
+// The first poll of a sum, sent right behind the block's own adds, met none of
+// a later block's, and the sum was seen a second way to L2 and back (700
+// cycles) after it.  A block now waits before it by what it was ahead of the
+// last block: kLeadUp cycles more after a poll that came too early, kLeadDown
+// less after one that served.  Fixed waits were best at 200 cycles on 17 blocks
+// and at 300 to 600 on 152, growing with the slices of a block; this follows
+// them, for each sum and block.  Milliseconds without, with 32/8, 64/8, 64/4
+// and 128/8: 64 x 32 mixed 1.95, 1.83, 1.83, 1.85, 1.91; 127 x 64 FP64 5.29,
+// 5.08, 5.02, 4.98, 5.00; 512 x 256 mixed 38.8, 38.6, 38.2, 38.2, 38.4; the
+// gradient at 255 x 128 10.65, 10.17, 9.95, 9.89, 10.10.  Two to four polls in
+// flight were slower (5 to 30 %), and so was a second line for every other
+// block's adds (0 to 5 %).
+constexpr unsigned kLeadUp = 64, kLeadDown = 4, kLeadMost = 1000;
 
 // 2^-E for the window |v| < 2^E of a sum whose last value was `last` (0:
 // none): E = 20 + its exponent.
@@ -323,11 +336,12 @@ struct ExactSum {
     unsigned long long* words;
     unsigned long long last[2][2 * kSumWords];  // the words at the end of the last sums
     unsigned half;
+    unsigned lead;  // cycles between the block's adds and its first poll
 
     __device__ __forceinline__ void init(void* area) {  // by one thread
         words = (unsigned long long*)area;
         for (int k = 0; k < 4 * kSumWords; k++) last[k / (2 * kSumWords)][k % (2 * kSumWords)] = 0;
-        half = 0;
+        half = lead = 0;
     }
     // The block's limbs are in sh; the sums of NV (1 or 2) values over the
     // grid's G <= 255 blocks, value 0 in the even lanes and value 1 in the odd
@@ -358,8 +372,11 @@ struct ExactSum {
             asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(add) : "memory");
         }
         out();
+        // no gain behind a fence (1M dof: 212.1 ms with and without)
+        unsigned wait = kFence ? 0 : lead;
+        for (const unsigned c0 = (unsigned)clock(); (unsigned)clock() - c0 < wait;) {}
         PollLimit lim;
-        for (;;) {
+        for (bool first = true;; first = false) {
             bool ok = true;
             if (lane < kW) {
                 if (kFence)  // not a fence behind the loop: it would wait for stores too
@@ -368,12 +385,18 @@ struct ExactSum {
                     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(d) : "l"(p) : "memory");
                 ok = ((d - before) >> 56) == G;
             }
-            if (__all_sync(0xffffffffu, ok)) break;
+            if (__all_sync(0xffffffffu, ok)) {
+                wait = first ? wait - min(wait, kLeadDown) : min(wait + kLeadUp, kLeadMost);
+                break;
+            }
             if (__any_sync(0xffffffffu, lim.expired(status))) return 2;
         }
         const long long t = (long long)((d - before) & ((1ull << 56) - 1)) - ((long long)G << 32);
         if (lane < kW) last[h][lane] = d;
-        if (lane == 0) half = h ^ 1;
+        if (lane == 0) {
+            half = h ^ 1;
+            lead = wait;
+        }
         // even lanes put value 0 together, odd ones value 1
         const uint32_t k = NV == 2 ? lane & 1 : 0;
         long long l[kSumWords];
