@@ -1511,7 +1511,7 @@ double slice_waves(const std::vector<uint32_t>& sp, double gamma, unsigned total
 // memory and L2; but a wave's block works for one system, however small.
 // Milliseconds in the other form and in waves: 24 systems of 48 and 96
 // elements' length 12.5 and 7.0, 6 of 96 and 192 25.0 and 11.1, 12 of 64 to 256
-// 50.0 and 30.3, 24 of 48 to 192 40.0 and 33.6, 24 of 64 to 512 277 and 259; 20 of
+// 50.0 and 30.3, 24 of 48 to 192 40.0 and 33.6, 24 of 64 to 512 277 and 259 (254 now); 20 of
 // 96 to 384, six of them of 2,323 slices, stay (180, in waves 196).
 bool best_waves(const std::vector<uint32_t>& sp, double gamma, unsigned nsm,
                 std::vector<Wave>& waves) {
