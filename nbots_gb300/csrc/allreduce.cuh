@@ -17,7 +17,7 @@
 // the previous value: the sum is exact but for each addend's bits below that,
 // closer than float-float or FP64 adds.  Where the window does not serve (no
 // previous value yet, an addend above it, infinities and NaN, a sum 2^30
-// times smaller than the last) every block sees so, and the records sum the
+// times smaller than the last, a float-float sum below 2^-97) every block sees so, and the records sum the
 // same values with float-float or FP64 adds instead.
 //
 // AllReduce: sums by records.  A record is 16 bytes, a 64-bit payload and a
@@ -278,13 +278,14 @@ struct ExactSum {
     // The block's limbs are in sh; the sums of NV (1 or 2) values over the
     // grid's G <= 255 blocks, value 0 in the even lanes and value 1 in the odd
     // ones (one value: in every lane), as an integer x of 61 bits and an
-    // exponent e: x 2^e.  kFence: the sum is also a barrier for the block's
+    // exponent e: x 2^e (least: as in read_limbs).  kFence: the sum is also a barrier for the block's
     // plain loads and stores (release before it, acquire after it).  out() is
     // called when the block's part is on its way.  Returns 0, 1 (outside the
     // window: sum again by records) or 2 (give up).  Called by one whole warp.
     template <int NV, bool kFence, class Out>
     __device__ __forceinline__ int sum(const int* sh, uint32_t n_warps, uint32_t G, int* status,
-                                       const int (&window)[NV], long long& x, int& e, Out out) {
+                                       const int (&window)[NV], int least, long long& x, int& e,
+                                       Out out) {
         const uint32_t lane = threadIdx.x & 31;
         constexpr uint32_t kW = NV * kSumWords;
         // lanes 0-15 add the even warps' words, lanes 16-31 the odd ones'
@@ -334,13 +335,13 @@ struct ExactSum {
         long long l[kSumWords];
 #pragma unroll
         for (int j = 0; j < kSumWords; j++) l[j] = __shfl_sync(0xffffffffu, t, k * kSumWords + j);
-        const bool bad = read_limbs(l, NV == 2 && k ? window[NV - 1] : window[0], x, e);
+        const bool bad = read_limbs(l, NV == 2 && k ? window[NV - 1] : window[0], least, x, e);
         return __any_sync(0xffffffffu, bad);
     }
     template <int NV>
     __device__ __forceinline__ int sum(const int* sh, uint32_t n_warps, uint32_t G, int* status,
-                                       const int (&window)[NV], long long& x, int& e) {
-        return sum<NV, false>(sh, n_warps, G, status, window, x, e, [] {});
+                                       const int (&window)[NV], int least, long long& x, int& e) {
+        return sum<NV, false>(sh, n_warps, G, status, window, least, x, e, [] {});
     }
 };
 

@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cg_bsr_slice(CgBsrArgs a, BsrSl
             if (warp == 0) {
                 long long xs;
                 int es;
-                const int st = sum1.sum<1>(s_sum1, nw, G, a.status, win, xs, es);
+                const int st = sum1.sum<1>(s_sum1, nw, G, a.status, win, kLeastF64, xs, es);
                 if (tid == 0) {
                     s_again = st;
                     if (!st) finish(exact_f64(xs, es));
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cg_bsr_slice(CgBsrArgs a, BsrSl
             if (warp == 0) {
                 long long xs;
                 int es;
-                const int st = sum2.sum<2>(s_sum2, nw, G, a.status, win, xs, es);
+                const int st = sum2.sum<2>(s_sum2, nw, G, a.status, win, kLeastF64, xs, es);
                 const double t = exact_f64(xs, es);  // g.q in lane 0, g.g in lane 1
                 const double gg = __shfl_sync(0xffffffffu, t, 1);
                 if (tid == 0) {

@@ -80,11 +80,17 @@ __device__ __forceinline__ void limbs_of(double v, int E, int (&l)[kSumWords]) {
     l[kLimbs] = out;
 }
 
+// The least exponent e of a sum x 2^e that exact_ff (exact_f64) reads: 2^(e + 31)
+// is a normal float.  A float-float sum then is at least 2^-97, below which its
+// low part would have no bits left.
+constexpr int kLeastFF = -126 - 31, kLeastF64 = -1000;
+
 // A sum's value from the sums l of its addends' limbs: an integer x of 61 bits
-// and an exponent e, x 2^e.  window: the exponent E of its limbs.  True: outside the
-// window, to be summed another way.
-__device__ __forceinline__ bool read_limbs(const long long (&l)[kSumWords], int window, long long& x,
-                                           int& e) {
+// and an exponent e, x 2^e.  window: the exponent E of its limbs; least: of kLeastFF
+// and kLeastF64 the one that the sum is read as.  True: outside the window, to be
+// summed another way.
+__device__ __forceinline__ bool read_limbs(const long long (&l)[kSumWords], int window, int least,
+                                           long long& x, int& e) {
     // carries: hi 2^60 + lo 2^20 + l4 units of 2^(E - 100)
     const long long l4 = l[4] & ((1 << kLimbBits) - 1);
     long long lo = (l[2] << kLimbBits) + l[3] + (l[4] >> kLimbBits);
@@ -97,11 +103,11 @@ __device__ __forceinline__ bool read_limbs(const long long (&l)[kSumWords], int 
     if (m >= 0) v = (hi << (40 + m)) + (lo << m) + (l4 >> (kLimbBits - m));
     else v = m >= -40 ? (hi << (40 + m)) + (lo >> -m) : hi >> (-m - 40);
     // a sum 2^30 times below the last one has too few bits left
-    const bool bad = l[kLimbs] != 0 || (m == kLimbBits && (v < 0 ? -v : v) < (1ll << 50));
+    const bool few = m == kLimbBits && (v < 0 ? -v : v) < (1ll << 50);
     const int up = max(__clzll(v < 0 ? ~v : v) - 3, 0);
     x = v << up;
     e = window - 4 * kLimbBits - m - up;
-    return bad;
+    return l[kLimbs] != 0 || few || e < least;
 }
 
 // x 2^e in FP64.
@@ -110,8 +116,7 @@ __device__ __forceinline__ double exact_f64(long long x, int e) {
     return __longlong_as_double(__double_as_longlong(__ll2double_rn(x)) + ((long long)e << 52));
 }
 
-// x 2^e as a float-float number (|x| < 2^61; |e| small enough that 2^(e + 62)
-// is a float): the leading 31 bits and the 31 below them, each exact in an
+// x 2^e as a float-float number (|x| < 2^61, e >= kLeastFF): the leading 31 bits and the 31 below them, each exact in an
 // integer register.
 __device__ __forceinline__ FF exact_ff(long long x, int e) {
     const int a = (int)(x >> 31);

@@ -384,7 +384,8 @@ __device__ __forceinline__ int mixed_sum(MixSums& m, ExactSum& site, int first, 
     if (threadIdx.x < 32) {
         long long x;
         int e;
-        const int st = site.sum<NV, kFence>(m.sh, blockDim.x >> 5, g.g_size, g.status, window, x, e,
+        const int st = site.sum<NV, kFence>(m.sh, blockDim.x >> 5, g.g_size, g.status, window,
+                                            kLeastFF, x, e,
                                             [] { if (kFence) bar_arrive(1); });
         FF t[NV];
         const FF mine = exact_ff(x, e);

@@ -330,7 +330,7 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
                 long long xs;
                 int es;
                 const int st =
-                    sum1.sum<1>(s_sum1, nw, G, g.status, {window_exponent(scale[0])}, xs, es);
+                    sum1.sum<1>(s_sum1, nw, G, g.status, {window_exponent(scale[0])}, kLeastFF, xs, es);
                 if (tid == 0) {
                     s_again = st;
                     if (!st) finish(exact_ff(xs, es));
@@ -381,7 +381,7 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
                 int es;
                 const int st = sum2.sum<2>(
                     s_sum2, nw, G, g.status,
-                    {window_exponent(scale[0]), window_exponent(scale[1])}, xs, es);
+                    {window_exponent(scale[0]), window_exponent(scale[1])}, kLeastFF, xs, es);
                 const FF t = exact_ff(xs, es);  // r.z in lane 0, |r|^2 in lane 1
                 const FF rrs = {__shfl_sync(0xffffffffu, t.hi, 1), __shfl_sync(0xffffffffu, t.lo, 1)};
                 if (tid == 0) {

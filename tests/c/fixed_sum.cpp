@@ -57,7 +57,7 @@ extern "C" int sum_ff(int n, const float* hi, const float* lo, float last, float
     }
     long long x;
     int e;
-    const bool bad = read_limbs(total, window_exponent(scale), x, e);
+    const bool bad = read_limbs(total, window_exponent(scale), kLeastFF, x, e);
     if (bad) return 1;
     const FF f = exact_ff(x, e);
     out[0] = f.hi;
@@ -75,7 +75,7 @@ extern "C" int sum_f64(int n, const double* v, double last, double* out) {
     }
     long long x;
     int e;
-    if (read_limbs(total, E, x, e)) return 1;
+    if (read_limbs(total, E, kLeastF64, x, e)) return 1;
     *out = exact_f64(x, e);
     return 0;
 }

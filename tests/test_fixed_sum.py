@@ -62,3 +62,17 @@ def test_values_outside_the_window_are_refused(lib, bad):
     assert lib.sum_ff(3, hi.ctypes.data, lo.ctypes.data, 1.0, out.ctypes.data) == 1
     d = C.c_double()
     assert lib.sum_f64(3, v.ctypes.data, 1.0, C.byref(d)) == 1
+
+
+# a last value down to the window's lower end, the next sum far below it: read
+# out as float-float, 2^-97 is the least (test_sums_are_right has the rest)
+@pytest.mark.parametrize("drop", range(12, 32))
+@pytest.mark.parametrize("ex", [-82, -81, -80, -79, -78, -75, -70, -67, -66, -65, -60])
+def test_float_float_sums_at_the_lower_end(lib, ex, drop):
+    rng = np.random.default_rng(1000 - 40 * ex + drop)
+    for sign in (1.0, -1.0):
+        v = sign * np.ldexp(rng.uniform(0.5, 1.0, 3) / 3, ex - drop)
+        bad, got, exact = sum_ff(lib, v, 2.0 ** ex)
+        assert bad or abs(got - exact) <= abs(exact) * Fraction(1, 2 ** 46)
+        if ex >= -80 and ex - drop >= -95 and drop <= 20:
+            assert not bad
