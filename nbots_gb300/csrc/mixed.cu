@@ -171,8 +171,8 @@ struct MixScalars {
         target2f = (float)target2;
         delta2 = (float)(a.delta * a.delta);
         rmax2 = (float)rr64;
-        converged = !(rr64 > target2);
-        return (converged || a.max_iter == 0) ? 2 : 0;
+        converged = rr64 <= target2;  // not where it is NaN
+        return (!(rr64 > target2) || a.max_iter == 0) ? 2 : 0;
     }
     __device__ __forceinline__ FF alpha(FF pw) const { return ff_div(rz, pw); }
     // The recursive residual's {r.z, |r|^2}: 1 when a reliable update is
@@ -200,8 +200,8 @@ struct MixScalars {
         rr64 = t[0];
         rmax2 = (float)rr64;
         nupd++;
-        converged = !(rr64 > target2);
-        const int stop = converged || k >= max_iter;
+        converged = rr64 <= target2;
+        const int stop = !(rr64 > target2) || k >= max_iter;
         if (!stop) {
             const FF rzn = ff_from_double(t[1]);
             beta = ff_div(rzn, rz);
