@@ -218,16 +218,19 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
         return {make_float2(v.x, v.y), make_float2(v.z, v.w)};
     };
     // r = b - A u in FP64 for this lane's row (float-float), z = r / Aii;
-    // |r|^2 in FP64, r.z; |b|^2, r.p.  A u in nbots' own arithmetic: the
-    // solve is judged on the residual that nb_sparse_multiply_vector gives
-    // for u.  Near the FP64 floor of a system the one with FMAs differs from
-    // it by a third of the tolerance.
+    // |r|^2 in FP64, r.z; |b|^2, r.p.  The iteration goes on with A u by FMAs,
+    // |r|^2 is of A u in nbots' own arithmetic: the solve is judged on the residual
+    // that nb_sparse_multiply_vector gives for u.  Near the FP64 floor of a system
+    // the two differ by a third of the tolerance, and the error of the rounded one
+    // is the larger by a fifth (64 x 32 lognormal: 2.2e-13 and 1.8e-13 of |b|).
     auto true_residual = [&](double& rr, FFAcc& rz, double* bb, double* rp) {
         if (!live) return;
-        const double2 au = spmv_row_f64<true>(a.A, s, lane, u);
+        double2 an;
+        const double2 au = spmv_row_f64<true>(a.A, s, lane, u, &an);
         const double2 bi = b[i];
         const double r0 = bi.x - au.x, r1 = bi.y - au.y;
-        rr = fma(r0, r0, fma(r1, r1, rr));
+        const double j0 = bi.x - an.x, j1 = bi.y - an.y;
+        rr = fma(j0, j0, fma(j1, j1, rr));
         if (bb) *bb = fma(bi.x, bi.x, fma(bi.y, bi.y, *bb));
         if (rp) *rp = dot_with(r0, r1, kGhost ? P[li] : as4(p), *rp);
         const FF f0 = ff_from_double(r0), f1 = ff_from_double(r1);

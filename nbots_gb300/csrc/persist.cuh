@@ -268,32 +268,33 @@ __device__ __forceinline__ void group_reduce0(const double* part, uint32_t G, do
     }
 }
 
-// (A x) for node row (s, lane) with FP64 values: FMAs, or (kRounded) nbots'
-// rounded products and left-to-right sums.
+// (A x) for node row (s, lane) with FP64 values and FMAs; kRounded: also in
+// *rounded with nbots' rounded products and left-to-right sums.
 template <bool kRounded = false>
 __device__ __forceinline__ double2 spmv_row_f64(const nbg_bsr_t& A, uint32_t s, uint32_t lane,
-                                                const double2* __restrict__ xv) {
+                                                const double2* __restrict__ xv,
+                                                double2* rounded = nullptr) {
     const double2* __restrict__ bv = reinterpret_cast<const double2*>(A.b64);
     // the 36 B/block matrix stream passes through L2 once per iteration;
     // evict_first keeps the vectors there (1M dof: 64.3 -> 62.8 us/iteration)
     const uint64_t pol = l2_policy(false);
-    double y0 = 0.0, y1 = 0.0;
+    double y0 = 0.0, y1 = 0.0, n0 = 0.0, n1 = 0.0;
     const uint32_t k0 = A.slice_off[s], k1 = A.slice_off[s + 1];
 #pragma unroll 3
     for (uint32_t k = k0; k < k1; k++) {
         const size_t e = (size_t)k * 32 + lane;
         const double2 xc = xv[ld_hint(A.bcol + e, pol)];
         const double2 top = ld_hint(bv + 2 * e, pol), bot = ld_hint(bv + 2 * e + 1, pol);
+        y0 = fma(top.x, xc.x, y0);
+        y0 = fma(top.y, xc.y, y0);
+        y1 = fma(bot.x, xc.x, y1);
+        y1 = fma(bot.y, xc.y, y1);
         if (kRounded) {
-            y0 = add(add(y0, mul(top.x, xc.x)), mul(top.y, xc.y));
-            y1 = add(add(y1, mul(bot.x, xc.x)), mul(bot.y, xc.y));
-        } else {
-            y0 = fma(top.x, xc.x, y0);
-            y0 = fma(top.y, xc.y, y0);
-            y1 = fma(bot.x, xc.x, y1);
-            y1 = fma(bot.y, xc.y, y1);
+            n0 = add(add(n0, mul(top.x, xc.x)), mul(top.y, xc.y));
+            n1 = add(add(n1, mul(bot.x, xc.x)), mul(bot.y, xc.y));
         }
     }
+    if (kRounded) *rounded = make_double2(n0, n1);
     return make_double2(y0, y1);
 }
 
