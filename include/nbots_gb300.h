@@ -310,7 +310,7 @@ typedef struct {
     uint32_t niter;        /* FP32 iterations */
     uint32_t n_updates;    /* FP64 residual recomputations */
     int status;            /* 0 converged, 1 not converged, < 0 error */
-    double relres;         /* final FP64 ||b - A x|| / ||b|| */
+    double relres;         /* final FP64 ||b - A x|| / ||b||, A x as nbg_spmv_csr_f64 gives it */
     double bnorm;
 } nbg_mixed_result_t;
 

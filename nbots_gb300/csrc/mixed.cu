@@ -25,7 +25,7 @@
 // & van der Vorst 1996) adds x to the FP64 solution and recomputes
 // r = b - A u in FP64 with the FP64 values whenever |r| has fallen by
 // `delta` since the last one; p is kept, so the Krylov progress survives.
-// Convergence is judged on the FP64 residual only.  Three grid barriers per
+// Convergence is judged on the FP64 residual only (row_residual).  Three grid barriers per
 // iteration in the global-gather form (L1 | L2 | L3 of
 // cg_precond_jacobi.c:50-74), two sums over the grid in the ghost-node form
 // below and in the slice form (mixed_slice.cuh): folding L3
@@ -175,33 +175,36 @@ struct MixScalars {
         return (!(rr64 > target2) || a.max_iter == 0) ? 2 : 0;
     }
     __device__ __forceinline__ FF alpha(FF pw) const { return ff_div(rz, pw); }
-    // The recursive residual's {r.z, |r|^2}: 1 when a reliable update is
-    // due, else 0 with beta.
+    // The recursive residual's {r.z, |r|^2}: when a reliable update is due 1, or
+    // 3 when the solve may end with it; else 0 with beta.
     __device__ __forceinline__ int step(FF rz_new, FF rr, uint32_t max_iter, FF& beta) {
         if (rr.hi > rmax2) rmax2 = rr.hi;
         k++;
-        const int upd = rr.hi <= delta2 * rmax2 || rr.hi <= target2f || k >= max_iter;
-        if (!upd) {
-            beta = ff_div(rz_new, rz);
-            rz = rz_new;
+        if (rr.hi <= 4.f * target2f || k >= max_iter) {
+            if (rr.hi <= target2f || rr.hi <= delta2 * rmax2 || k >= max_iter) return 3;
+        } else if (rr.hi <= delta2 * rmax2) {
+            return 1;
         }
-        return upd;
+        beta = ff_div(rz_new, rz);
+        rz = rz_new;
+        return 0;
     }
     // A reliable update's {|r|^2, r.z, r.p} (FP64), r the recomputed residual
-    // and p the last direction: 2 stop, else 0 with beta.  The recursive
+    // and p the last direction: 2 stop, else 0 with beta.  judged: |r|^2 is the
+    // one that the solve is judged on (row_residual).  The recursive
     // residual was orthogonal to p, the recomputed one is only up to the
     // rounding of b - A u.  Near the FP64 floor of a system r.(z + beta p)
     // then differs from r.z, and with r.z as the next step's numerator the
     // error stayed in every later step until the iteration diverged (the
     // 20,000-point T3 L-shape at relres 8e-12: 36 after 40,000 iterations).
     // From a relative difference of `least` on the step takes r.(z + beta p).
-    __device__ __forceinline__ int replaced(const double (&t)[3], uint32_t max_iter, FF& beta,
-                                            float least = 0.f) {
+    __device__ __forceinline__ int replaced(const double (&t)[3], bool judged, uint32_t max_iter,
+                                            FF& beta, float least = 0.f) {
         rr64 = t[0];
         rmax2 = (float)rr64;
         nupd++;
-        converged = rr64 <= target2;
-        const int stop = !(rr64 > target2) || k >= max_iter;
+        converged = judged && rr64 <= target2;
+        const int stop = converged || rr64 != rr64 || k >= max_iter;
         if (!stop) {
             const FF rzn = ff_from_double(t[1]);
             beta = ff_div(rzn, rz);
@@ -309,27 +312,43 @@ __device__ __forceinline__ double dot_with(double r0, double r1, float4 p, doubl
     return fma(r0, (double)p.x + (double)p.z, fma(r1, (double)p.y + (double)p.w, rp));
 }
 
-// r = b - A u in FP64 for the own rows, stored as float-float; z = r / Aii
+// r = b - A u in FP64 of node row i (s, lane), A u by FMAs: the iteration goes on
+// with it.  Accumulates |r|^2 and optionally |b|^2.  judge: |r|^2 is of A u in
+// nbots' own arithmetic, the residual that nb_sparse_multiply_vector gives for
+// u, on which every form of the solver is judged.  Near the FP64 floor of a system
+// the two differ by a third of the tolerance, and the error of the rounded one is
+// the larger by a fifth (64 x 32 lognormal: 2.2e-13 and 1.8e-13 of |b|).  Its
+// FP64 operations, two for each FMA, are spent where the solve may end only.
+__device__ __forceinline__ double2 row_residual(const MixArgs& a, uint32_t s, uint32_t lane,
+                                                bool judge, double& rr, double* bb) {
+    const uint32_t i = s * 32 + lane;
+    const double2* __restrict__ u = reinterpret_cast<const double2*>(a.u);
+    const double2 bi = reinterpret_cast<const double2*>(a.b)[i];
+    double2 an;
+    const double2 au = judge ? spmv_row_f64<true>(a.A, s, lane, u, &an)
+                             : spmv_row_f64(a.A, s, lane, u);
+    if (!judge) an = au;
+    const double j0 = bi.x - an.x, j1 = bi.y - an.y;
+    rr = fma(j0, j0, fma(j1, j1, rr));
+    if (bb) *bb = fma(bi.x, bi.x, fma(bi.y, bi.y, *bb));
+    return make_double2(bi.x - au.x, bi.y - au.y);
+}
+
+// r = b - A u for the own rows (row_residual), stored as float-float; z = r / Aii
 // (float-float); accumulates |r|^2 (FP64), r.z and optionally |b|^2 and r.p;
 // with set_p, p = z (own copy and the global one).
 template <int kThreads>
 __device__ __forceinline__ void true_residual(const MixArgs& a, const Own& o, uint32_t s0,
-                                              uint32_t s1, double& rr, FFAcc& rz, double* bb,
-                                              double* rp, bool set_p) {
+                                              uint32_t s1, bool judge, double& rr, FFAcc& rz,
+                                              double* bb, double* rp, bool set_p) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t nw = kThreads / 32;
-    const double2* __restrict__ u = reinterpret_cast<const double2*>(a.u);
-    const double2* __restrict__ b = reinterpret_cast<const double2*>(a.b);
     for (uint32_t s = s0 + warp; s < s1; s += nw) {
         const uint32_t i = s * 32 + lane, li = i - s0 * 32;
         if (i >= a.A.Nn) continue;
-        const double2 au = spmv_row_f64(a.A, s, lane, u);
-        const double2 bi = b[i];
-        const double r0 = bi.x - au.x, r1 = bi.y - au.y;
-        rr = fma(r0, r0, fma(r1, r1, rr));
-        if (bb) *bb = fma(bi.x, bi.x, fma(bi.y, bi.y, *bb));
-        if (rp) *rp = dot_with(r0, r1, o.p[li], *rp);
-        const FF f0 = ff_from_double(r0), f1 = ff_from_double(r1);
+        const double2 ri = row_residual(a, s, lane, judge, rr, bb);
+        if (rp) *rp = dot_with(ri.x, ri.y, o.p[li], *rp);
+        const FF f0 = ff_from_double(ri.x), f1 = ff_from_double(ri.y);
         o.r[li] = make_float4(f0.hi, f1.hi, f0.lo, f1.lo);
         const float2 di = o.dv[li];
         const FF z0 = ff_mulf(f0, di.x), z1 = ff_mulf(f1, di.y);
@@ -441,7 +460,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
     __shared__ double red[3 * 32];
     float2* const ffred = reinterpret_cast<float2*>(red);
     __shared__ float s_alpha[2], s_beta[2];
-    __shared__ int s_flag;  // 0 iterate, 1 reliable update, 2 stop
+    __shared__ int s_flag;  // 0 iterate, 1 reliable update, 2 stop, 3 update and judge
     __shared__ MixScalars sc;  // thread 0 only
     const unsigned G = g.g_size;
     const uint32_t rank = blockIdx.x - g.g_base;
@@ -472,7 +491,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
         __syncwarp();
         double rrl = 0.0, bbl = 0.0;
         FFAcc rzk{0.f, 0.f};
-        true_residual<kThreads>(a, o, s0, s1, rrl, rzk, &bbl, nullptr, true);
+        true_residual<kThreads>(a, o, s0, s1, true, rrl, rzk, &bbl, nullptr, true);
         const FF t = rzk.result();
         double v[3] = {rrl, bbl, (double)t.hi + (double)t.lo};
         group_publish<3>(v, red, part2, rank);
@@ -573,7 +592,8 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
         }
         if (s_flag) {
             // reliable update: u += x in FP64, then r = b - A u in FP64
-            double2* __restrict__ u = reinterpret_cast<double2*>(a.u);
+            const bool judge = s_flag == 3;
+            double2* const u = reinterpret_cast<double2*>(a.u);
             for (uint32_t s = s0 + warp; s < s1; s += nw) {
                 const uint32_t i = s * 32 + lane, li = i - s0 * 32;
                 if (i >= Nn) continue;
@@ -587,7 +607,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
             if (sync()) goto done;
             double rrl = 0.0, rpl = 0.0;
             FFAcc rzk{0.f, 0.f};
-            true_residual<kThreads>(a, o, s0, s1, rrl, rzk, nullptr, &rpl, false);
+            true_residual<kThreads>(a, o, s0, s1, judge, rrl, rzk, nullptr, &rpl, false);
             const FF t = rzk.result();
             double v[3] = {rrl, (double)t.hi + (double)t.lo, rpl};
             group_publish<3>(v, red, part2, rank);
@@ -597,7 +617,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
             if (threadIdx.x == 0) {
                 FF be;
                 // rows in global memory: the large systems, far from their floor
-                s_flag = sc.replaced(tt, a.max_iter, be, kRes ? 0.f : 1e-7f);
+                s_flag = sc.replaced(tt, judge, a.max_iter, be, kRes ? 0.f : 1e-7f);
                 if (!s_flag) {
                     s_beta[0] = be.hi;
                     s_beta[1] = be.lo;
@@ -824,23 +844,17 @@ __device__ __forceinline__ float4* ghost_x(const MixArgs& a) { return a.x4; }
 template <int kThreads>
 __device__ __forceinline__ void true_residual_ghost(const MixArgs& a, float4* r4, const float4* P,
                                                     float4* Z, uint32_t s0, uint32_t s1,
-                                                    double& rr, FFAcc& rz, double* bb,
-                                                    double* rp) {
+                                                    bool judge, double& rr, FFAcc& rz,
+                                                    double* bb, double* rp) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t nw = kThreads / 32;
-    const double2* __restrict__ u = reinterpret_cast<const double2*>(a.u);
-    const double2* __restrict__ b = reinterpret_cast<const double2*>(a.b);
     const float2* __restrict__ dinv = reinterpret_cast<const float2*>(a.A.dinv32);
     for (uint32_t s = s0 + warp; s < s1; s += nw) {
         const uint32_t i = s * 32 + lane, li = i - s0 * 32;
         if (i >= a.A.Nn) continue;
-        const double2 au = spmv_row_f64(a.A, s, lane, u);
-        const double2 bi = b[i];
-        const double r0 = bi.x - au.x, r1 = bi.y - au.y;
-        rr = fma(r0, r0, fma(r1, r1, rr));
-        if (bb) *bb = fma(bi.x, bi.x, fma(bi.y, bi.y, *bb));
-        if (rp) *rp = dot_with(r0, r1, P[li], *rp);
-        const FF f0 = ff_from_double(r0), f1 = ff_from_double(r1);
+        const double2 ri = row_residual(a, s, lane, judge, rr, bb);
+        if (rp) *rp = dot_with(ri.x, ri.y, P[li], *rp);
+        const FF f0 = ff_from_double(ri.x), f1 = ff_from_double(ri.y);
         r4[i] = make_float4(f0.hi, f1.hi, f0.lo, f1.lo);
         const float2 di = dinv[i];
         const FF z0 = ff_mulf(f0, di.x), z1 = ff_mulf(f1, di.y);
@@ -856,7 +870,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
     __shared__ double red[3 * 32];
     float2* const ffred = reinterpret_cast<float2*>(red);
     __shared__ float s_alpha[2], s_beta[2];
-    __shared__ int s_flag;  // 0 iterate, 1 reliable update, 2 stop
+    __shared__ int s_flag;  // 0 iterate, 1 reliable update, 2 stop, 3 update and judge
     __shared__ MixScalars sc;  // thread 0 only
     __shared__ MixSums ms;
     const unsigned G = g.g_size;
@@ -905,7 +919,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
         }
         double rrl = 0.0, bbl = 0.0;
         FFAcc rzk{0.f, 0.f};
-        true_residual_ghost<kThreads>(a, r4, P, P, s0, s1, rrl, rzk, &bbl, nullptr);
+        true_residual_ghost<kThreads>(a, r4, P, P, s0, s1, true, rrl, rzk, &bbl, nullptr);
         const FF t = rzk.result();
         double v[3] = {rrl, bbl, (double)t.hi + (double)t.lo};
         group_publish<3>(v, red, part2, rank);
@@ -1019,7 +1033,8 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
         }
         if (s_flag) {
             // reliable update: u += x in FP64, then r = b - A u in FP64
-            double2* __restrict__ u = reinterpret_cast<double2*>(a.u);
+            const bool judge = s_flag == 3;
+            double2* const u = reinterpret_cast<double2*>(a.u);
             for (uint32_t s = s0 + warp; s < s1; s += nw) {
                 const uint32_t i = s * 32 + lane;
                 if (i >= Nn) continue;
@@ -1033,7 +1048,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
             if (sync()) goto done;
             double rrl = 0.0, rpl = 0.0;
             FFAcc rzk{0.f, 0.f};
-            true_residual_ghost<kThreads>(a, r4, P, W, s0, s1, rrl, rzk, nullptr, &rpl);
+            true_residual_ghost<kThreads>(a, r4, P, W, s0, s1, judge, rrl, rzk, nullptr, &rpl);
             const FF t = rzk.result();
             double v[3] = {rrl, (double)t.hi + (double)t.lo, rpl};
             group_publish<3>(v, red, part2, rank);
@@ -1042,7 +1057,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
             group_reduce0<3>(part2, G, tt);
             if (tid == 0) {
                 FF be;
-                s_flag = sc.replaced(tt, a.max_iter, be);
+                s_flag = sc.replaced(tt, judge, a.max_iter, be);
                 if (!s_flag) {
                     s_beta[0] = be.hi;
                     s_beta[1] = be.lo;

@@ -123,7 +123,7 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
     __shared__ uint64_t s_ff[2 * 32];
     __shared__ float s_alpha[2], s_beta[2];
     __shared__ float s_scale[3];  // windows of p.w, r.z, |r|^2
-    __shared__ int s_flag;  // 0 iterate, 1 reliable update, 2 stop, 3 give up
+    __shared__ int s_flag;  // 0 iterate, 1 reliable update, 2 stop, 3 update and judge
     __shared__ int s_fail;   // a wait for ghosts or records ran out
     __shared__ int s_again;  // the fixed-point sum's status: 1 sum by records, 2 give up
     __shared__ MixScalars sc;  // thread 0 only
@@ -159,7 +159,7 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
     unsigned char* const zy = zx + (size_t)Nn * 16;
     double* const part0 = g.part;
     double* const part2 = g.part + 3 * g.pstride;
-    double2* __restrict__ u = reinterpret_cast<double2*>(a.u);
+    double2* const u = reinterpret_cast<double2*>(a.u);
     const double2* __restrict__ b = reinterpret_cast<const double2*>(a.b);
     auto area = [&]() { return kBatch ? g.sums - kArBytes : sl.ar; };
     unsigned bar_target = 0;
@@ -217,23 +217,13 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
     auto from4 = [](float4 v) -> FF2 {
         return {make_float2(v.x, v.y), make_float2(v.z, v.w)};
     };
-    // r = b - A u in FP64 for this lane's row (float-float), z = r / Aii;
-    // |r|^2 in FP64, r.z; |b|^2, r.p.  The iteration goes on with A u by FMAs,
-    // |r|^2 is of A u in nbots' own arithmetic: the solve is judged on the residual
-    // that nb_sparse_multiply_vector gives for u.  Near the FP64 floor of a system
-    // the two differ by a third of the tolerance, and the error of the rounded one
-    // is the larger by a fifth (64 x 32 lognormal: 2.2e-13 and 1.8e-13 of |b|).
-    auto true_residual = [&](double& rr, FFAcc& rz, double* bb, double* rp) {
+    // r = b - A u for this lane's row (row_residual) as float-float, z = r / Aii;
+    // |r|^2 in FP64, r.z; |b|^2, r.p
+    auto true_residual = [&](bool judge, double& rr, FFAcc& rz, double* bb, double* rp) {
         if (!live) return;
-        double2 an;
-        const double2 au = spmv_row_f64<true>(a.A, s, lane, u, &an);
-        const double2 bi = b[i];
-        const double r0 = bi.x - au.x, r1 = bi.y - au.y;
-        const double j0 = bi.x - an.x, j1 = bi.y - an.y;
-        rr = fma(j0, j0, fma(j1, j1, rr));
-        if (bb) *bb = fma(bi.x, bi.x, fma(bi.y, bi.y, *bb));
-        if (rp) *rp = dot_with(r0, r1, kGhost ? P[li] : as4(p), *rp);
-        const FF f0 = ff_from_double(r0), f1 = ff_from_double(r1);
+        const double2 ri = row_residual(a, s, lane, judge, rr, bb);
+        if (rp) *rp = dot_with(ri.x, ri.y, kGhost ? P[li] : as4(p), *rp);
+        const FF f0 = ff_from_double(ri.x), f1 = ff_from_double(ri.y);
         r = {make_float2(f0.hi, f1.hi), make_float2(f0.lo, f1.lo)};
         const FF2 z = ff2_mulf(r, di);
         rz.fma2(r.hi.x, r.lo.x, z.hi.x, z.lo.x);
@@ -278,7 +268,7 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
     {   // init: x = 0, r = b - A u (FP64), p = z
         double rrl = 0.0, bbl = 0.0;
         FFAcc rzk{0.f, 0.f};
-        true_residual(rrl, rzk, &bbl, nullptr);
+        true_residual(true, rrl, rzk, &bbl, nullptr);
         p = ff2_mulf(r, di);
         if (kXGlobal && live) a.x4[i] = as4(x);
         if (kGhost) {
@@ -419,6 +409,7 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
         }
         if (s_flag) {
             // reliable update: u += x in FP64, then r = b - A u in FP64
+            const bool judge = s_flag == 3;
             if (live) {
                 if (kXGlobal) x = from4(a.x4[i]);
                 double2 ui = u[i];
@@ -431,7 +422,7 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
             if (sync()) goto done;
             double rrl = 0.0, rpl = 0.0;
             FFAcc rzk{0.f, 0.f};
-            true_residual(rrl, rzk, nullptr, &rpl);
+            true_residual(judge, rrl, rzk, nullptr, &rpl);
             const FF t = rzk.result();
             double v[3] = {rrl, (double)t.hi + (double)t.lo, rpl};
             group_publish<3>(v, red, part2, rank);
@@ -440,7 +431,7 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
             group_reduce0<3>(part2, G, tt);
             if (tid == 0) {
                 FF be;
-                s_flag = sc.replaced(tt, a.max_iter, be);
+                s_flag = sc.replaced(tt, judge, a.max_iter, be);
                 if (!s_flag) {
                     s_beta[0] = be.hi;
                     s_beta[1] = be.lo;
