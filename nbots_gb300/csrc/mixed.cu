@@ -197,9 +197,12 @@ struct MixScalars {
     // then differs from r.z, and with r.z as the next step's numerator the
     // error stayed in every later step until the iteration diverged (the
     // 20,000-point T3 L-shape at relres 8e-12: 36 after 40,000 iterations).
-    // From a relative difference of `least` on the step takes r.(z + beta p).
+    // From a relative difference of kOffLeast on the step takes r.(z + beta p);
+    // smaller ones do not show (13 models, Q4 and T3, from 1e-6 to 1e-11: the same
+    // iterations, to 1 %, with 0 and 1e-7, and closer to the floor either one ahead).
+    static constexpr float kOffLeast = 1e-7f;
     __device__ __forceinline__ int replaced(const double (&t)[3], bool judged, uint32_t max_iter,
-                                            FF& beta, float least = 0.f) {
+                                            FF& beta) {
         rr64 = t[0];
         rmax2 = (float)rr64;
         nupd++;
@@ -210,7 +213,7 @@ struct MixScalars {
             beta = ff_div(rzn, rz);
             rz = rzn;
             const FF off = ff_mul(beta, ff_from_double(t[2]));
-            if (!(fabsf(off.hi) <= least * rzn.hi)) {
+            if (!(fabsf(off.hi) <= kOffLeast * rzn.hi)) {
                 const FF rp = ff_add(rzn, off);
                 if (rp.hi > 0.1f * rzn.hi) rz = rp;
                 else beta = FF{0.f, 0.f};  // p points uphill: start again from z
@@ -448,13 +451,10 @@ __device__ __forceinline__ int mixed_sum(MixSums& m, ExactSum& site, int first, 
 // scalar recurrences (step lengths, residual norms, stopping and update
 // decisions) run in thread 0 (MixScalars) and reach the block through
 // shared memory as FP32 pairs and flags.
-template <int kOwn, int kThreads>
+// kExact: sums in fixed point, else by partials.
+template <int kOwn, int kThreads, bool kExact>
 __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, unsigned char* smem) {
     constexpr bool kRes = kOwn == 3;
-    // with resident rows the single-system launch sums in fixed point, as the
-    // ghost-node form; rows in global memory leave it bound by DRAM, and
-    // batched launches give each system a few blocks: by partials there
-    constexpr bool kExact = kThreads == kMixThreads && kRes;
     constexpr int kRB = kThreads == kMixThreads ? kReduceBatch : 1;
     __shared__ std::conditional_t<kExact, MixSums, NoMixSums> ms;
     __shared__ double red[3 * 32];
@@ -616,8 +616,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
             group_reduce0<3>(part2, G, tt);
             if (threadIdx.x == 0) {
                 FF be;
-                // rows in global memory: the large systems, far from their floor
-                s_flag = sc.replaced(tt, judge, a.max_iter, be, kRes ? 0.f : 1e-7f);
+                s_flag = sc.replaced(tt, judge, a.max_iter, be);
                 if (!s_flag) {
                     s_beta[0] = be.hi;
                     s_beta[1] = be.lo;
@@ -673,15 +672,16 @@ done:
 
 // kOwn: the own-row vectors in dynamic shared memory (known at compile time,
 // so their addresses are 32-bit shared ones).
-template <int kOwn>
+template <int kOwn, bool kExact>
 __global__ void __launch_bounds__(kMixThreads, kMixMinBlocks) k_cg_mixed(MixArgs a,
                                                                                 Group g) {
     extern __shared__ __align__(16) unsigned char smem[];
-    mixed_solve<kOwn, kMixThreads>(a, g, smem);
+    mixed_solve<kOwn, kMixThreads, kExact>(a, g, smem);
 }
 
 // Many independent systems stored in one block-diagonal layout, in one
-// launch: block b works for system groups[block_of[b]].
+// launch: block b works for system groups[block_of[b]].  A system has a few
+// blocks: sums by partials.
 template <int kOwn>
 __global__ void __launch_bounds__(kBatThreads, kBatMinBlocks)
     k_cg_mixed_many(MixArgs a, const Group* __restrict__ groups,
@@ -690,7 +690,7 @@ __global__ void __launch_bounds__(kBatThreads, kBatMinBlocks)
     __shared__ Group sg;
     if (threadIdx.x == 0) sg = groups[block_of[blockIdx.x]];
     __syncthreads();
-    mixed_solve<kOwn, kBatThreads>(a, sg, smem);
+    mixed_solve<kOwn, kBatThreads, false>(a, sg, smem);
 }
 
 // The SpMV's matrix stream (FP32 values, remainders, columns: 32 B per block
@@ -1228,11 +1228,25 @@ int slice_setup(const nbg_bsr_t& A, unsigned G, int threads, char* plan, cudaStr
 }  // namespace
 
 namespace {
-const void* mixed_kernel(int own) {
-    return own == 3 ? (const void*)k_cg_mixed<3>
-         : own == 2 ? (const void*)k_cg_mixed<2>
-         : own == 1 ? (const void*)k_cg_mixed<1>
-                    : (const void*)k_cg_mixed<0>;
+// Whether the rows of a block, without any ghosts, would fit in the ghost-node
+// form's shared memory (2.1M dof on 152 SMs).  Up to there the global-gather form
+// sums in fixed point as that form does, so that both give the same bits with any
+// workspace; past it by partials, its iterations being bound by DRAM (us with
+// partials and in fixed point, own rows in global memory: 1.13M dof 44.4 and 44.9,
+// 1.67M 63.6 and 64.7, 1.97M 72.1 and 72.5; the ghost-node form itself at 1.13M dof
+// 37.6 and 34.5, at 1.28M 42.1 and 39.2).
+bool ghost_sizes(uint32_t n_slices, int nsm) {
+    size_t most = 0;
+    const unsigned G = std::max(1u, (unsigned)nsm * kMixMinBlocks);
+    return allow_smem((const void*)k_cg_mixed_ghost, &most) == cudaSuccess &&
+           (n_slices + G - 1) / G * (size_t)(32 * 2 * sizeof(float4)) <= most;
+}
+
+const void* mixed_kernel(int own, bool exact) {
+    return own == 3 ? (const void*)k_cg_mixed<3, true>
+         : own == 2 ? (const void*)k_cg_mixed<2, true>
+         : own == 1 ? (exact ? (const void*)k_cg_mixed<1, true> : (const void*)k_cg_mixed<1, false>)
+                    : (const void*)k_cg_mixed<0, false>;
 }
 
 // slices per block of a batch's waves
@@ -1331,7 +1345,7 @@ extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint
         // as many of the own rows' vectors in shared memory as fit, at the
         // same grid: the rows of a block, and so the sums, are the same
         for (int own = NBG_MIXED_RESIDENT ? 3 : 0; own >= 0 && rc == NBG_OK && !fn; own--) {
-            fn = mixed_kernel(own);
+            fn = mixed_kernel(own, ghost_sizes(A->n_slices, nsm));
             rc = coop_grid_resident(fn, A->n_slices, own_node_bytes(own) * 32, &G, &dyn, kMixThreads,
                                     kMixMinBlocks);
             a.resident = own == 3;
