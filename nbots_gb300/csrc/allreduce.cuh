@@ -15,10 +15,11 @@
 // Integer sums do not depend on their order, so the result is the same bits
 // whatever the partition.  The window reaches from 2^20 above to 2^-80 below
 // the previous value: the sum is exact but for each addend's bits below that,
-// closer than float-float or FP64 adds.  Where the window does not serve (no
-// previous value yet, an addend above it, infinities and NaN, a sum 2^30
-// times smaller than the last, a float-float sum below 2^-97) every block sees so, and the records sum the
-// same values with float-float or FP64 adds instead.
+// half a unit of 2^-80 times the previous value, within the bounds of float-float
+// and FP64 adds.  Where the window does not serve (no previous value yet, an
+// addend above it, infinities and NaN, a sum 2^24 times smaller than the last, a
+// float-float sum below 2^-97) every block sees so, and the records sum the same
+// values with float-float or FP64 adds instead.
 //
 // AllReduce: sums by records.  A record is 16 bytes, a 64-bit payload and a
 // 64-bit epoch, written and read as one 128-bit access

@@ -14,7 +14,7 @@
 //   - p of the rows and of the block's ghosts and as many entries of each row
 //     as fit stay in shared memory (ghost_plan.cuh);
 //   - sums over the grid are taken in fixed point in one hop (allreduce.cuh),
-//     off the FP64 pipe; they are closer than FP64 adds;
+//     off the FP64 pipe;
 //   - owners publish q = g / Aii as epoch-tagged records, which the warps
 //     that do not sum poll meanwhile; every block then updates its ghosts' p
 //     itself, as mixed.cu's ghost-node form does.

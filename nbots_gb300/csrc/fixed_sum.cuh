@@ -102,8 +102,10 @@ __device__ __forceinline__ bool read_limbs(const long long (&l)[kSumWords], int 
     long long v;
     if (m >= 0) v = (hi << (40 + m)) + (lo << m) + (l4 >> (kLimbBits - m));
     else v = m >= -40 ? (hi << (40 + m)) + (lo >> -m) : hi >> (-m - 40);
-    // a sum 2^30 times below the last one has too few bits left
-    const bool few = m == kLimbBits && (v < 0 ? -v : v) < (1ll << 50);
+    // every addend is rounded to half a unit: n addends to n 2^-57 of a sum that is
+    // 2^24 times below the last one, under the bound of a sum by FP64 adds (n 2^-53);
+    // a smaller one has too few bits left
+    const bool few = m == kLimbBits && (v < 0 ? -v : v) < (1ll << 56);
     const int up = max(__clzll(v < 0 ? ~v : v) - 3, 0);
     x = v << up;
     e = window - 4 * kLimbBits - m - up;

@@ -76,3 +76,16 @@ def test_float_float_sums_at_the_lower_end(lib, ex, drop):
         assert bad or abs(got - exact) <= abs(exact) * Fraction(1, 2 ** 46)
         if ex >= -80 and ex - drop >= -95 and drop <= 20:
             assert not bad
+
+
+# 100,000 equal addends just below half a unit (2^-80 of the last sum) above a
+# whole one: every one is rounded the same way.  What is given is within the bound
+# of a sum by FP64 adds, (n - 1) 2^-53 of itself.
+@pytest.mark.parametrize("drop", range(20, 32))
+def test_sums_that_fall_far_keep_fp64_accuracy(lib, drop):
+    n = 100_000
+    k = 2 ** (80 - drop) // n
+    v = np.full(n, (k + 0.49) * 2.0 ** -80)
+    bad, got, exact = sum_f64(lib, v, 1.0)
+    assert bad or abs(got - exact) <= exact * Fraction(n - 1, 2 ** 53)
+    assert not bad or drop > 23
