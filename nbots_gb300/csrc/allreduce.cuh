@@ -222,7 +222,6 @@ __device__ __forceinline__ void block_sum_end(typename S::T (&v)[NV], const uint
 // words of one site: [2 epochs][2 values * kSumWords], each epoch a 128-byte
 // line of its own; zero at launch
 constexpr size_t kExactBytes = 2 * 128;
-constexpr unsigned kExactMaxBlocks = 255;  // counted in a byte
 // The first poll of a sum, sent right behind the block's own adds, met none of
 // a later block's, and the sum was seen a second way to L2 and back (700
 // cycles) after it.  A block now waits before it by what it was ahead of the

@@ -384,7 +384,7 @@ int bsr_slice_setup(const nbg_bsr_t& A, bool jac, bool lagged, char* plan, cudaS
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
             cudaSuccess)
         return 0;
-    const unsigned most = std::min((unsigned)nsm, kExactMaxBlocks);
+    const unsigned most = exact_grid((unsigned)nsm);
     if (A.n_slices > 32 * most) return 0;
     *G = std::min(most, (A.n_slices + 1) / 2);
     const unsigned spb = (A.n_slices + *G - 1) / *G;

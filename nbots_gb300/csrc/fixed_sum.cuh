@@ -12,6 +12,12 @@ namespace nbg {
 
 constexpr int kLimbs = 5, kLimbBits = 20;
 constexpr int kSumWords = kLimbs + 1;  // per value: the limbs, values outside the window
+// Blocks of a launch that sums in fixed point: they are counted in the top byte of
+// a word, and a count past 255 would never be complete.
+constexpr unsigned kExactMaxBlocks = 255;
+constexpr unsigned exact_grid(unsigned blocks) {
+    return blocks < kExactMaxBlocks ? blocks : kExactMaxBlocks;
+}
 
 // 2^-E for the window |v| < 2^E of a sum whose last value was `last` (0:
 // none): E = 20 + its exponent.

@@ -1184,7 +1184,7 @@ int ghost_setup(const nbg_bsr_t& A, unsigned G, char* plan, cudaStream_t s, Ghos
 // and 24 slices per block: 4,290 dof 4.5, 4.4, 4.4, 5.5, 8.5; 16,770 dof
 // 4.5, 4.4, 4.9, 5.9, 8.9.
 unsigned slice_grid(uint32_t n_slices, int nsm) {
-    const unsigned most = std::min((unsigned)nsm, kExactMaxBlocks);
+    const unsigned most = exact_grid((unsigned)nsm);
     if (n_slices > most * (kMixThreads / 32)) return 0;
     return std::min(most, (n_slices + 3) / 4);
 }
@@ -1237,7 +1237,7 @@ namespace {
 // 37.6 and 34.5, at 1.28M 42.1 and 39.2).
 bool ghost_sizes(uint32_t n_slices, int nsm) {
     size_t most = 0;
-    const unsigned G = std::max(1u, (unsigned)nsm * kMixMinBlocks);
+    const unsigned G = exact_grid((unsigned)nsm * kMixMinBlocks);
     return allow_smem((const void*)k_cg_mixed_ghost, &most) == cudaSuccess &&
            (n_slices + G - 1) / G * (size_t)(32 * 2 * sizeof(float4)) <= most;
 }
@@ -1336,7 +1336,7 @@ extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint
     } else if (e == cudaSuccess && plan) {
         // one block per SM, as the resident global-gather form's first choice
         const unsigned want = (A->n_slices + kMixThreads / 32 - 1) / (kMixThreads / 32);
-        G = std::max(1u, std::min((unsigned)nsm * kMixMinBlocks, want));
+        G = std::max(1u, std::min(exact_grid((unsigned)nsm * kMixMinBlocks), want));
         ghost = ghost_setup(*A, G, plan, s, &gh, &dyn) == 1;
         (void)cudaGetLastError();
         if (ghost) fn = (const void*)k_cg_mixed_ghost;
@@ -1347,7 +1347,7 @@ extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint
         for (int own = NBG_MIXED_RESIDENT ? 3 : 0; own >= 0 && rc == NBG_OK && !fn; own--) {
             fn = mixed_kernel(own, ghost_sizes(A->n_slices, nsm));
             rc = coop_grid_resident(fn, A->n_slices, own_node_bytes(own) * 32, &G, &dyn, kMixThreads,
-                                    kMixMinBlocks);
+                                    kMixMinBlocks, kExactMaxBlocks);
             a.resident = own == 3;
             if (own > 0 && (dyn == 0 || (own < 3 && dyn > kOwnSmem))) fn = nullptr;
         }
@@ -1552,7 +1552,7 @@ bool best_waves(const std::vector<uint32_t>& sp, double gamma, unsigned nsm,
     for (uint32_t most : {kSlicesFew, kSlicesMost}) {
         std::vector<Wave> w;
         const double cost =
-            NBG_MIXED_RESIDENT ? slice_waves(sp, gamma, std::min(nsm, kExactMaxBlocks), most, w) : -1.0;
+            NBG_MIXED_RESIDENT ? slice_waves(sp, gamma, exact_grid(nsm), most, w) : -1.0;
         if (cost >= 0.0 && cost < best) {
             best = cost;
             waves.swap(w);

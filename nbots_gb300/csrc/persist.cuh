@@ -335,10 +335,11 @@ inline cudaError_t allow_smem(const void* fn, size_t* most) {
 // data per slice in dynamic shared memory: the largest blocks-per-SM count
 // (min_blocks, then fewer) at which every block's slices fit.  *dyn = 0
 // means they do not fit even at one block per SM and the kernel must keep
-// those rows in global memory.
+// those rows in global memory.  At most `most_blocks` blocks then.
 inline int coop_grid_resident(const void* fn, uint32_t n_slices, size_t bytes_per_slice,
                               unsigned* G, size_t* dyn, int threads = kPersistThreads,
-                              int min_blocks = kPersistMinBlocks) {
+                              int min_blocks = kPersistMinBlocks,
+                              unsigned most_blocks = kMaxBlocks) {
     int dev = 0, nsm = 0;
     size_t most = 0;
     NBG_CHECK(cudaGetDevice(&dev));
@@ -347,6 +348,7 @@ inline int coop_grid_resident(const void* fn, uint32_t n_slices, size_t bytes_pe
     const unsigned want = (n_slices + threads / 32 - 1) / (threads / 32);
     for (int per_sm = min_blocks; bytes_per_slice && per_sm >= 1; --per_sm) {
         unsigned g = (unsigned)nsm * (unsigned)per_sm;
+        if (most_blocks < g) g = most_blocks;
         if (want < g) g = want;
         if (g < 1) g = 1;
         const size_t spb = (n_slices + g - 1) / g;

@@ -79,3 +79,12 @@ extern "C" int sum_f64(int n, const double* v, double last, double* out) {
     *out = exact_f64(x, e);
     return 0;
 }
+
+// Whether the grid chosen for `blocks` blocks counts itself: each adds one to the
+// top byte of a word that may hold anything before.
+extern "C" int grid_counts(unsigned blocks, unsigned long long before) {
+    const unsigned G = exact_grid(blocks);
+    unsigned long long d = before;
+    for (unsigned b = 0; b < G; b++) d += 1ull << 56;
+    return G >= 1 && G <= blocks && (d - before) >> 56 == G;
+}

@@ -89,3 +89,10 @@ def test_sums_that_fall_far_keep_fp64_accuracy(lib, drop):
     bad, got, exact = sum_f64(lib, v, 1.0)
     assert bad or abs(got - exact) <= exact * Fraction(n - 1, 2 ** 53)
     assert not bad or drop > 23
+
+
+def test_every_grid_counts_itself(lib):
+    lib.grid_counts.argtypes = [C.c_uint, C.c_ulonglong]
+    for blocks in (1, 2, 152, 254, 255, 256, 257, 304, 511, 512, 608):
+        for before in (0, 200 << 56, 255 << 56 | 12345):
+            assert lib.grid_counts(blocks, before)
