@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_cg_bsr_slice(CgBsrArgs a, BsrSl
     uint16_t* const MC = reinterpret_cast<uint16_t*>(M1 + cap);
     const uint32_t m0 = ls * per + r;
     const double2* __restrict__ b = reinterpret_cast<const double2*>(a.b);
-    double2* __restrict__ gx = reinterpret_cast<double2*>(a.x);
+    double2* const gx = reinterpret_cast<double2*>(a.x);  // read here, written through a.x
     unsigned bar_target = 0;
     auto sync = [&]() { return grid_barrier_count(a.bar, G, bar_target, a.status); };
     uint64_t qepoch = 1;

@@ -470,7 +470,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
     group_slice_range(g.s_begin, g.s_end, rank, G, s0, s1);
     const uint32_t Nn = a.A.Nn;
     const Own o = own_vectors<kOwn>(a, smem, s0, (s1 - s0) * 32);
-    float4* __restrict__ gp = a.p;
+    float4* const gp = a.p;
     double* const part0 = g.part;
     double* const part1 = g.part + g.pstride;
     double* const part2 = g.part + 3 * g.pstride;
