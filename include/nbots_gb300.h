@@ -290,7 +290,7 @@ size_t nbg_cg_bsr_workspace_bytes(uint32_t N);
 /* With this much (more: a 16-bit local column per layout entry and per-block
  * ghost lists) systems of up to 32 slices per SM take the slice form, which
  * keeps its vectors in registers and its rows' and ghosts' p in shared memory;
- * ws NULL allocates this size. */
+ * ws NULL allocates this size.  The same as the other for larger systems. */
 size_t nbg_cg_bsr_layout_workspace_bytes(const nbg_bsr_t *A);
 int nbg_cg_bsr_f64(const nbg_bsr_t *A, const double *b, double *x, uint32_t max_iter,
                    double tol, unsigned flags, nbg_cg_result_t *result, void *ws,

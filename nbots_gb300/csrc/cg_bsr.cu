@@ -316,7 +316,7 @@ size_t cg_bsr_bytes(uint32_t N) { return cg_bsr_core_bytes(N) + perm_tail_bytes(
 extern "C" size_t nbg_cg_bsr_workspace_bytes(uint32_t N) { return cg_bsr_bytes(N); }
 
 extern "C" size_t nbg_cg_bsr_layout_workspace_bytes(const nbg_bsr_t* A) {
-    return A ? cg_bsr_bytes(A->N) + ghost_plan_bytes(*A) : 0;
+    return A ? cg_bsr_bytes(A->N) + slice_plan_bytes(*A) : 0;
 }
 
 extern "C" int nbg_cg_bsr_f64(const nbg_bsr_t* A, const double* b, double* x, uint32_t max_iter,
@@ -327,12 +327,18 @@ extern "C" int nbg_cg_bsr_f64(const nbg_bsr_t* A, const double* b, double* x, ui
     if (A->Nn == 0) return NBG_OK;
     if (!A->b64 || ((flags & NBG_CG_JACOBI) && !A->dinv64)) return NBG_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t need = cg_bsr_bytes(A->N), plan_bytes = ghost_plan_bytes(*A);
+    const size_t need = cg_bsr_bytes(A->N), plan_bytes = slice_plan_bytes(*A);
     void* own = nullptr;
     if (!ws) {
-        NBG_CHECK(cudaMalloc(&own, need + plan_bytes));
-        ws = own;
         ws_bytes = need + plan_bytes;
+        cudaError_t e = cudaMalloc(&own, ws_bytes);
+        if (e == cudaErrorMemoryAllocation && plan_bytes) {  // the global form needs no plan
+            (void)cudaGetLastError();
+            ws_bytes = need;
+            e = cudaMalloc(&own, ws_bytes);
+        }
+        NBG_CHECK(e);
+        ws = own;
     } else if (ws_bytes < need) {
         return NBG_ERR_ARG;
     }

@@ -369,6 +369,15 @@ const void* bsr_slice_kernel_of(int dofs, int threads) {
                           : (const void*)k_cg_bsr_slice<JAC, LAGGED, 2, 1024>;
 }
 
+// Workspace of the slice form's plan; none for a system that is too large for it.
+size_t slice_plan_bytes(const nbg_bsr_t& A) {
+    int dev = 0, nsm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0;
+    return A.n_slices > 32 * exact_grid((unsigned)nsm) ? 0 : ghost_plan_bytes(A);
+}
+
 // Launch data of the slice form: 1, or 0 (the global form runs).  Two slices
 // per block, one warp per scheduler, while there are SMs (4,290 dof: 4.9 us
 // per iteration with 2 slices, 5.5 with 4; 16,770 dof: 5.1 and 5.7).  A lane

@@ -1815,11 +1815,16 @@ extern "C" int nbg_mixed_batch_create(nbg_mixed_batch_t** out, const nbg_bsr_t* 
     int dev = 0, nsm = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const bool slices = e == cudaSuccess && best_waves(m->slice_ptr, 1.5, (unsigned)nsm, waves);
+    bool slices = e == cudaSuccess && best_waves(m->slice_ptr, 1.5, (unsigned)nsm, waves);
     const size_t base_bytes = batch_bytes(A->N, n_sys), sums = align256((size_t)n_sys * kBatchSums),
                  ranges = align256(sizeof(uint2) * kMaxBlocks);
     const size_t need = base_bytes + (slices ? sums + ranges + ghost_plan_bytes(*A) : 0);
     if (e == cudaSuccess) e = cudaMalloc(&m->ws, need);
+    if (e == cudaErrorMemoryAllocation && slices) {  // side by side needs no plan
+        (void)cudaGetLastError();
+        slices = false;
+        e = cudaMalloc(&m->ws, base_bytes);
+    }
     if (e != cudaSuccess) {
         delete m;
         return nbg_cuda_error(e);
