@@ -216,9 +216,9 @@ int nbg_solver_multiply(nbg_solver_t *s, const double *in, double *out)
 				      s->stream);
 	if (rc == NBG_OK && !direct)
 		rc = nbg_d2h(out, s->b, 8 * (size_t)s->N, s->stream);
-	if (rc == NBG_OK)
-		rc = nbg_stream_sync(s->stream);
-	return rc;
+	/* also after an error: what was launched may still read in */
+	const int done = nbg_stream_sync(s->stream);
+	return rc != NBG_OK ? rc : done;
 }
 
 int nbg_solver_device_csr(nbg_solver_t *s, const uint32_t **row_ptr, const uint32_t **col_idx,

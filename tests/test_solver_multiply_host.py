@@ -1,0 +1,19 @@
+"""nbg_solver_multiply (host/solve.c) against stand-ins of the device calls
+(tests/c/solver_multiply.c): no launched kernel may still read the caller's vector
+after it has returned, also when a launch failed.  CPU only."""
+import os
+import subprocess
+
+from conftest import ROOT
+
+
+def test_multiply_waits_also_after_an_error(tmp_path):
+    from nbots_gb300 import _lib as L
+    L.lib()  # built
+    pkg, exe = os.path.dirname(L.GPU_SO), tmp_path / "solver_multiply"
+    subprocess.run(["gcc", "-std=c99", "-Wall", "-I" + os.path.join(ROOT, "include"),
+                    "-I" + os.path.join(ROOT, "nbots_gb300", "host"),
+                    os.path.join(ROOT, "tests", "c", "solver_multiply.c"), "-o", str(exe),
+                    "-L" + pkg, "-lnbots_gpu", "-lnbots_host", "-Wl,-rpath," + pkg], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0 and r.stdout == "ok\n", r.returncode
