@@ -1875,6 +1875,26 @@ extern "C" uint32_t nbg_mixed_batch_blocks(const nbg_mixed_batch_t* m, uint32_t*
     return m->G;
 }
 
+// How the last launch ran, for checks: the return value is its waves of the slice
+// form (0: all systems side by side, < 0: error), form[i] is NBG_MIXED_GHOST where
+// system i had its ghosts in shared memory, else NBG_MIXED_RESIDENT_ROWS or
+// NBG_MIXED_GLOBAL_ROWS.
+extern "C" int nbg_mixed_batch_form(const nbg_mixed_batch_t* m, int* form) {
+    if (!m || !form) return NBG_ERR_ARG;
+    std::vector<unsigned char> state((size_t)m->n_sys * kStateStride);
+    NBG_CHECK(cudaMemcpyAsync(state.data(), m->d_state, state.size(), cudaMemcpyDeviceToHost,
+                              m->stream));
+    NBG_CHECK(cudaStreamSynchronize(m->stream));
+    for (uint32_t i = 0; i < m->n_sys; i++) {
+        int failed;
+        memcpy(&failed, &state[i * kStateStride + 128 + 4 * kNoPlan], sizeof(int));
+        form[i] = m->own == kSliceForm && !failed ? NBG_MIXED_GHOST
+                : m->own >= 3                     ? NBG_MIXED_RESIDENT_ROWS
+                                                  : NBG_MIXED_GLOBAL_ROWS;
+    }
+    return (int)m->waves.size();
+}
+
 extern "C" int nbg_mixed_batch_set_sensitivity(nbg_mixed_batch_t* m, uint32_t nen,
                                                uint32_t N_elem, const double* nod,
                                                const uint32_t* conn, double nu, double thickness,
