@@ -103,7 +103,6 @@ struct MixArgs {
     uint32_t max_iter;
     double tol, delta;
     unsigned flags;
-    int resident;      // own-row vectors live in shared memory
     uint32_t keep;     // share of each block's matrix stream kept in L2, of 2^32 (all ones: all)
 };
 
@@ -385,9 +384,7 @@ struct MixSums {
     }
 };
 
-struct NoMixSums {
-    float scale[3];
-};
+struct NoMixSums {};
 
 template <int NV, bool kFence, class Sync, class Finish, class Meanwhile>
 __device__ __forceinline__ int mixed_sum(MixSums& m, ExactSum& site, int first, FF (&v)[NV],
@@ -502,8 +499,10 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
         group_reduce0<3>(part2, G, t);
         if (threadIdx.x == 0) {
             s_flag = sc.start(t, a);
-            ms.scale[1] = window_scale(sc.rz.hi);
-            ms.scale[2] = window_scale((float)sc.rr64);
+            if constexpr (kExact) {
+                ms.scale[1] = window_scale(sc.rz.hi);
+                ms.scale[2] = window_scale((float)sc.rr64);
+            }
         }
         __syncthreads();
     }
@@ -1325,7 +1324,7 @@ extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const unsigned slice_g = NBG_MIXED_RESIDENT ? slice_grid(A->n_slices, nsm) : 0;
     const void* fn = nullptr;
-    a.resident = 1;
+    bool resident = slice_g != 0;  // the own rows' vectors on chip
     if (e == cudaSuccess && slice_g) {
         G = slice_g;
         threads = 32 * (int)((A->n_slices + G - 1) / G);
@@ -1348,7 +1347,7 @@ extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint
             fn = mixed_kernel(own, ghost_sizes(A->n_slices, nsm));
             rc = coop_grid_resident(fn, A->n_slices, own_node_bytes(own) * 32, &G, &dyn, kMixThreads,
                                     kMixMinBlocks, kExactMaxBlocks);
-            a.resident = own == 3;
+            resident = own == 3;
             if (own > 0 && (dyn == 0 || (own < 3 && dyn > kOwnSmem))) fn = nullptr;
         }
     }
@@ -1358,8 +1357,9 @@ extern "C" int nbg_cg_mixed(const nbg_bsr_t* A, const double* b, double* x, uint
     g.g_size = G;
     g.pstride = kMaxBlocks;
     if (ghost) a.keep = keep_share(*A, 30.0);
-    g_mixed_form = ghost ? NBG_MIXED_GHOST : slice_g || a.resident ? NBG_MIXED_RESIDENT_ROWS
-                                                                  : NBG_MIXED_GLOBAL_ROWS;
+    g_mixed_form = ghost      ? NBG_MIXED_GHOST
+                 : resident ? NBG_MIXED_RESIDENT_ROWS
+                            : NBG_MIXED_GLOBAL_ROWS;
     if (e == cudaSuccess && rc == NBG_OK) {
         void* args[] = {&a, &g, &gh, &sl};
         e = cudaLaunchCooperativeKernel(fn, dim3(G), dim3(threads), args, dyn, s);
@@ -1445,10 +1445,6 @@ size_t batch_bytes(uint32_t N, uint32_t n_sys) {
            align256((size_t)n_sys * kResStride * 8) + align256((size_t)n_sys * sizeof(Group)) +
            align256((size_t)kMaxBlocks * 4);
 }
-
-// Vector slots of the workspace shared by every system (indexed by the
-// global node row).
-void bind_vectors(MixArgs& a, char* base, uint32_t N) { carve_vectors(a, base, N); }
 
 double* part_slots(char* base, uint32_t N) {
     const size_t f = align256((size_t)N * 4), h = align256((size_t)N * 4);
@@ -1649,7 +1645,7 @@ int batch_plan(nbg_mixed_batch* m, double gamma) {
     a.A = m->A;
     a.b = m->b;
     a.u = m->x;
-    bind_vectors(a, base, m->A.N);
+    carve_vectors(a, base, m->A.N);  // shared by every system, by the global node row
     a.max_iter = m->max_iter;
     a.tol = m->tol;
     a.delta = m->delta;
@@ -1659,7 +1655,6 @@ int batch_plan(nbg_mixed_batch* m, double gamma) {
     // 351 with a fifth; 12 systems, 41 MB: 33.2 ms with all, 34.2 with none)
     const double in_l2 = stream_over_l2(m->A);
     a.keep = own == kSliceForm || (in_l2 > 0.0 && in_l2 <= 0.30) ? 0xFFFFFFFFu : 0;
-    a.resident = own >= 3;
     m->own = own;
     std::vector<Group> groups(n);
     std::vector<uint32_t> map(G);
