@@ -27,7 +27,7 @@ namespace {
 // bytes on a Q4 mesh; read by one lane per row they were 32 lines per load),
 // then writes the layout's arrays, every one coalesced.  The remainders'
 // counts take integer work (rem23_encode), so the fill is bound by its bytes:
-// 1M dof, 302 MB written and 190 read, 0.65 ms before and 0.13 now.  Slices
+// 1M dof, 302 MB written and 190 read, 0.65 ms before and 0.17 now.  Slices
 // wider than kFillCols read the CSR directly.
 constexpr int kFillWarps = 4, kFillCols = 12;
 

@@ -20,10 +20,8 @@
 //     itself, as mixed.cu's ghost-node form does.
 // The iteration, its stop rules and the check on the true residual are those
 // of the global form.  Microseconds per iteration, the global form and this
-// one: 4,290 dof 15.7 and 5.0, 16,770 dof 17.8 and 5.2, 66,306 dof 18.0 and
-// 7.4, 263,682 dof 27.2 and 16.7 (there FP64 issue bounds both).
-// With the sums' polls behind a lead (kLeadUp in allreduce.cuh, measured later)
-// the solves took 6 % less at 16,640 dof and 3.7 % less at 91,204.
+// one: 4,290 dof 15.7 and 4.9, 16,770 dof 17.8 and 4.9, 66,306 dof 18.0 and
+// 6.9, 263,682 dof 27.2 and 16.1 (there FP64 issue bounds both).
 
 struct BsrSliceArgs {
     GhostArgs gh;
@@ -384,7 +382,8 @@ size_t slice_plan_bytes(const nbg_bsr_t& A) {
 // per dof up to four slices per block, where the FP64 latency of a row counts
 // (16,770 dof: 5.1 us against 6.2 with a lane per row); above, its rounding up
 // of odd entry counts costs more FP64 issue than it saves (66,306 dof: 7.5
-// against 7.2, T3 with 91,204 dof: 9.1 against 8.3).
+// against 7.2, T3 with 91,204 dof: 9.1 against 8.3).  These with sums that were
+// polled at once, 0.1 to 0.3 us slower than with kLeadUp (allreduce.cuh).
 int bsr_slice_setup(const nbg_bsr_t& A, bool jac, bool lagged, char* plan, cudaStream_t s,
                     BsrSliceArgs* sl, const void** fn, unsigned* G, int* threads, size_t* dyn) {
     int dev = 0, nsm = 0, optin = 0;

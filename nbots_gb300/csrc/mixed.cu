@@ -1180,8 +1180,9 @@ int ghost_setup(const nbg_bsr_t& A, unsigned G, char* plan, cudaStream_t s, Ghos
 // block, one warp per scheduler, while there are SMs: the sums cost about
 // the same over 17 blocks as over 152, the SpMV's FP32 work grows with the
 // warps that share a scheduler.  Microseconds per iteration with 2, 4, 8, 16
-// and 24 slices per block: 4,290 dof 4.5, 4.4, 4.4, 5.5, 8.5; 16,770 dof
-// 4.5, 4.4, 4.9, 5.9, 8.9.
+// and 24 slices per block, with sums that were polled at once (0.3 slower than
+// with kLeadUp): 4,290 dof 4.5, 4.4, 4.4, 5.5, 8.5; 16,770 dof 4.5, 4.4, 4.9, 5.9,
+// 8.9.
 unsigned slice_grid(uint32_t n_slices, int nsm) {
     const unsigned most = exact_grid((unsigned)nsm);
     if (n_slices > most * (kMixThreads / 32)) return 0;

@@ -21,12 +21,10 @@
 //     poll their block's ghosts meanwhile.
 // An iteration has no barrier and no fence.  Microseconds per iteration, the
 // ghost-node form (one 1024-thread block per 32 slices) before and this one:
-// 4,290 dof 11.5 and 4.1, 66,306 dof 13.2 and 4.8, 91,204 dof (T3) 13.4 and
-// 5.1, 263,682 dof 14.0 and 8.9.  At 66,306 dof the rest is the two sums (2.2
+// 4,290 dof 11.5 and 4.1, 66,306 dof 13.2 and 4.6, 91,204 dof (T3) 13.4 and
+// 4.9, 263,682 dof 14.0 and 9.0.  At 66,306 dof the rest is the two sums (2.2
 // to 2.8 thousand cycles each, of which about 1,500 are the way to L2 and
-// back), the SpMV (2.1) and the two divisions (0.9).  With the sums' polls
-// behind a lead (kLeadUp in allreduce.cuh, measured later) the solves took 5 %
-// less at 4,290 dof, 7 at 66,048 and 1.7 at 263,682.
+// back), the SpMV (2.1) and the two divisions (0.9).
 //
 // kGhost = false (a workspace without the ghost plan, or ghosts that do not
 // fit): p is gathered from global memory and exchanged behind a barrier, the
