@@ -151,13 +151,14 @@ struct MixScalars {
     FF rz;                          // r.z of the current residual
     double rr64, bb, target2;       // true |r|^2, |b|^2, stopping threshold
     float rmax2, target2f, delta2;  // update test
+    float last;                     // recursive |r|^2 at the last update
     uint32_t k, nupd;
     int converged;
 
     __device__ __forceinline__ void clear() {
         rz = FF{0.f, 0.f};
         rr64 = bb = target2 = 0.0;
-        rmax2 = target2f = delta2 = 0.f;
+        rmax2 = target2f = delta2 = last = 0.f;
         k = nupd = 0;
         converged = 0;
     }
@@ -174,19 +175,24 @@ struct MixScalars {
         return (!(rr64 > target2) || a.max_iter == 0) ? 2 : 0;
     }
     __device__ __forceinline__ FF alpha(FF pw) const { return ff_div(rz, pw); }
-    // The recursive residual's {r.z, |r|^2}: when a reliable update is due 1, or
-    // 3 when the solve may end with it; else 0 with beta.
+    // The recursive residual's {r.z, |r|^2}: 1 when a reliable update is
+    // due, else 0 with beta.
     __device__ __forceinline__ int step(FF rz_new, FF rr, uint32_t max_iter, FF& beta) {
         if (rr.hi > rmax2) rmax2 = rr.hi;
         k++;
-        if (rr.hi <= 4.f * target2f || k >= max_iter) {
-            if (rr.hi <= target2f || rr.hi <= delta2 * rmax2 || k >= max_iter) return 3;
-        } else if (rr.hi <= delta2 * rmax2) {
-            return 1;
+        const int upd = rr.hi <= delta2 * rmax2 || rr.hi <= target2f || k >= max_iter;
+        if (!upd) {
+            beta = ff_div(rz_new, rz);
+            rz = rz_new;
+        } else {
+            last = rr.hi;
         }
-        beta = ff_div(rz_new, rz);
-        rz = rz_new;
-        return 0;
+        return upd;
+    }
+    // Whether the solve may end with the update that step() asked for; from every
+    // thread of the block.
+    __device__ __forceinline__ bool judge(uint32_t max_iter) const {
+        return last <= 4.f * target2f || k >= max_iter;
     }
     // A reliable update's {|r|^2, r.z, r.p} (FP64), r the recomputed residual
     // and p the last direction: 2 stop, else 0 with beta.  judged: |r|^2 is the
@@ -457,8 +463,8 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
     __shared__ double red[3 * 32];
     float2* const ffred = reinterpret_cast<float2*>(red);
     __shared__ float s_alpha[2], s_beta[2];
-    __shared__ int s_flag;  // 0 iterate, 1 reliable update, 2 stop, 3 update and judge
-    __shared__ MixScalars sc;  // thread 0 only
+    __shared__ int s_flag;  // 0 iterate, 1 reliable update, 2 stop
+    __shared__ MixScalars sc;  // thread 0 only, but for judge()
     const unsigned G = g.g_size;
     const uint32_t rank = blockIdx.x - g.g_base;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -591,7 +597,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
         }
         if (s_flag) {
             // reliable update: u += x in FP64, then r = b - A u in FP64
-            const bool judge = s_flag == 3;
+            const bool judge = sc.judge(a.max_iter);
             double2* const u = reinterpret_cast<double2*>(a.u);
             for (uint32_t s = s0 + warp; s < s1; s += nw) {
                 const uint32_t i = s * 32 + lane, li = i - s0 * 32;
@@ -869,8 +875,8 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
     __shared__ double red[3 * 32];
     float2* const ffred = reinterpret_cast<float2*>(red);
     __shared__ float s_alpha[2], s_beta[2];
-    __shared__ int s_flag;  // 0 iterate, 1 reliable update, 2 stop, 3 update and judge
-    __shared__ MixScalars sc;  // thread 0 only
+    __shared__ int s_flag;  // 0 iterate, 1 reliable update, 2 stop
+    __shared__ MixScalars sc;  // thread 0 only, but for judge()
     __shared__ MixSums ms;
     const unsigned G = g.g_size;
     const uint32_t rank = blockIdx.x - g.g_base;
@@ -1032,7 +1038,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
         }
         if (s_flag) {
             // reliable update: u += x in FP64, then r = b - A u in FP64
-            const bool judge = s_flag == 3;
+            const bool judge = sc.judge(a.max_iter);
             double2* const u = reinterpret_cast<double2*>(a.u);
             for (uint32_t s = s0 + warp; s < s1; s += nw) {
                 const uint32_t i = s * 32 + lane;

@@ -121,10 +121,10 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
     __shared__ uint64_t s_ff[2 * 32];
     __shared__ float s_alpha[2], s_beta[2];
     __shared__ float s_scale[3];  // windows of p.w, r.z, |r|^2
-    __shared__ int s_flag;  // 0 iterate, 1 reliable update, 2 stop, 3 update and judge
+    __shared__ int s_flag;  // 0 iterate, 1 reliable update, 2 stop
     __shared__ int s_fail;   // a wait for ghosts or records ran out
     __shared__ int s_again;  // the fixed-point sum's status: 1 sum by records, 2 give up
-    __shared__ MixScalars sc;  // thread 0 only
+    __shared__ MixScalars sc;  // thread 0 only, but for judge()
     const unsigned G = kBatch ? g.g_size : gridDim.x;
     const uint32_t rank = kBatch ? blockIdx.x - g.g_base : blockIdx.x;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -407,7 +407,7 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
         }
         if (s_flag) {
             // reliable update: u += x in FP64, then r = b - A u in FP64
-            const bool judge = s_flag == 3;
+            const bool judge = sc.judge(a.max_iter);
             if (live) {
                 if (kXGlobal) x = from4(a.x4[i]);
                 double2 ui = u[i];
