@@ -191,11 +191,11 @@ struct MixScalars {
     }
     // Whether the solve may end with the update that step() asked for; from every
     // thread of the block.
-    __device__ __forceinline__ bool judge(uint32_t max_iter) const {
+    __device__ __forceinline__ bool may_end(uint32_t max_iter) const {
         return last <= 4.f * target2f || k >= max_iter;
     }
     // A reliable update's {|r|^2, r.z, r.p} (FP64), r the recomputed residual
-    // and p the last direction: 2 stop, else 0 with beta.  judged: |r|^2 is the
+    // and p the last direction: 2 stop, else 0 with beta.  checked: |r|^2 is the
     // one that the solve is judged on (row_residual).  The recursive
     // residual was orthogonal to p, the recomputed one is only up to the
     // rounding of b - A u.  Near the FP64 floor of a system r.(z + beta p)
@@ -206,12 +206,12 @@ struct MixScalars {
     // smaller ones do not show (13 models, Q4 and T3, from 1e-6 to 1e-11: the same
     // iterations, to 1 %, with 0 and 1e-7, and closer to the floor either one ahead).
     static constexpr float kOffLeast = 1e-7f;
-    __device__ __forceinline__ int replaced(const double (&t)[3], bool judged, uint32_t max_iter,
+    __device__ __forceinline__ int replaced(const double (&t)[3], bool checked, uint32_t max_iter,
                                             FF& beta) {
         rr64 = t[0];
         rmax2 = (float)rr64;
         nupd++;
-        converged = judged && rr64 <= target2;
+        converged = checked && rr64 <= target2;
         const int stop = converged || rr64 != rr64 || k >= max_iter;
         if (!stop) {
             const FF rzn = ff_from_double(t[1]);
@@ -321,21 +321,21 @@ __device__ __forceinline__ double dot_with(double r0, double r1, float4 p, doubl
 }
 
 // r = b - A u in FP64 of node row i (s, lane), A u by FMAs: the iteration goes on
-// with it.  Accumulates |r|^2 and optionally |b|^2.  judge: |r|^2 is of A u in
+// with it.  Accumulates |r|^2 and optionally |b|^2.  check: |r|^2 is of A u in
 // nbots' own arithmetic, the residual that nb_sparse_multiply_vector gives for
 // u, on which every form of the solver is judged.  Near the FP64 floor of a system
 // the two differ by a third of the tolerance, and the error of the rounded one is
 // the larger by a fifth (64 x 32 lognormal: 2.2e-13 and 1.8e-13 of |b|).  Its
 // FP64 operations, two for each FMA, are spent where the solve may end only.
 __device__ __forceinline__ double2 row_residual(const MixArgs& a, uint32_t s, uint32_t lane,
-                                                bool judge, double& rr, double* bb) {
+                                                bool check, double& rr, double* bb) {
     const uint32_t i = s * 32 + lane;
     const double2* __restrict__ u = reinterpret_cast<const double2*>(a.u);
     const double2 bi = reinterpret_cast<const double2*>(a.b)[i];
     double2 an;
-    const double2 au = judge ? spmv_row_f64<true>(a.A, s, lane, u, &an)
+    const double2 au = check ? spmv_row_f64<true>(a.A, s, lane, u, &an)
                              : spmv_row_f64(a.A, s, lane, u);
-    if (!judge) an = au;
+    if (!check) an = au;
     const double j0 = bi.x - an.x, j1 = bi.y - an.y;
     rr = fma(j0, j0, fma(j1, j1, rr));
     if (bb) *bb = fma(bi.x, bi.x, fma(bi.y, bi.y, *bb));
@@ -347,14 +347,14 @@ __device__ __forceinline__ double2 row_residual(const MixArgs& a, uint32_t s, ui
 // with set_p, p = z (own copy and the global one).
 template <int kThreads>
 __device__ __forceinline__ void true_residual(const MixArgs& a, const Own& o, uint32_t s0,
-                                              uint32_t s1, bool judge, double& rr, FFAcc& rz,
+                                              uint32_t s1, bool check, double& rr, FFAcc& rz,
                                               double* bb, double* rp, bool set_p) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t nw = kThreads / 32;
     for (uint32_t s = s0 + warp; s < s1; s += nw) {
         const uint32_t i = s * 32 + lane, li = i - s0 * 32;
         if (i >= a.A.Nn) continue;
-        const double2 ri = row_residual(a, s, lane, judge, rr, bb);
+        const double2 ri = row_residual(a, s, lane, check, rr, bb);
         if (rp) *rp = dot_with(ri.x, ri.y, o.p[li], *rp);
         const FF f0 = ff_from_double(ri.x), f1 = ff_from_double(ri.y);
         o.r[li] = make_float4(f0.hi, f1.hi, f0.lo, f1.lo);
@@ -464,7 +464,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
     float2* const ffred = reinterpret_cast<float2*>(red);
     __shared__ float s_alpha[2], s_beta[2];
     __shared__ int s_flag;  // 0 iterate, 1 reliable update, 2 stop
-    __shared__ MixScalars sc;  // thread 0 only, but for judge()
+    __shared__ MixScalars sc;  // thread 0 only, but for may_end()
     const unsigned G = g.g_size;
     const uint32_t rank = blockIdx.x - g.g_base;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -597,7 +597,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
         }
         if (s_flag) {
             // reliable update: u += x in FP64, then r = b - A u in FP64
-            const bool judge = sc.judge(a.max_iter);
+            const bool check = sc.may_end(a.max_iter);
             double2* const u = reinterpret_cast<double2*>(a.u);
             for (uint32_t s = s0 + warp; s < s1; s += nw) {
                 const uint32_t i = s * 32 + lane, li = i - s0 * 32;
@@ -612,7 +612,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
             if (sync()) goto done;
             double rrl = 0.0, rpl = 0.0;
             FFAcc rzk{0.f, 0.f};
-            true_residual<kThreads>(a, o, s0, s1, judge, rrl, rzk, nullptr, &rpl, false);
+            true_residual<kThreads>(a, o, s0, s1, check, rrl, rzk, nullptr, &rpl, false);
             const FF t = rzk.result();
             double v[3] = {rrl, (double)t.hi + (double)t.lo, rpl};
             group_publish<3>(v, red, part2, rank);
@@ -621,7 +621,7 @@ __device__ __forceinline__ void mixed_solve(const MixArgs& a, const Group& g, un
             group_reduce0<3>(part2, G, tt);
             if (threadIdx.x == 0) {
                 FF be;
-                s_flag = sc.replaced(tt, judge, a.max_iter, be);
+                s_flag = sc.replaced(tt, check, a.max_iter, be);
                 if (!s_flag) {
                     s_beta[0] = be.hi;
                     s_beta[1] = be.lo;
@@ -849,7 +849,7 @@ __device__ __forceinline__ float4* ghost_x(const MixArgs& a) { return a.x4; }
 template <int kThreads>
 __device__ __forceinline__ void true_residual_ghost(const MixArgs& a, float4* r4, const float4* P,
                                                     float4* Z, uint32_t s0, uint32_t s1,
-                                                    bool judge, double& rr, FFAcc& rz,
+                                                    bool check, double& rr, FFAcc& rz,
                                                     double* bb, double* rp) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t nw = kThreads / 32;
@@ -857,7 +857,7 @@ __device__ __forceinline__ void true_residual_ghost(const MixArgs& a, float4* r4
     for (uint32_t s = s0 + warp; s < s1; s += nw) {
         const uint32_t i = s * 32 + lane, li = i - s0 * 32;
         if (i >= a.A.Nn) continue;
-        const double2 ri = row_residual(a, s, lane, judge, rr, bb);
+        const double2 ri = row_residual(a, s, lane, check, rr, bb);
         if (rp) *rp = dot_with(ri.x, ri.y, P[li], *rp);
         const FF f0 = ff_from_double(ri.x), f1 = ff_from_double(ri.y);
         r4[i] = make_float4(f0.hi, f1.hi, f0.lo, f1.lo);
@@ -876,7 +876,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
     float2* const ffred = reinterpret_cast<float2*>(red);
     __shared__ float s_alpha[2], s_beta[2];
     __shared__ int s_flag;  // 0 iterate, 1 reliable update, 2 stop
-    __shared__ MixScalars sc;  // thread 0 only, but for judge()
+    __shared__ MixScalars sc;  // thread 0 only, but for may_end()
     __shared__ MixSums ms;
     const unsigned G = g.g_size;
     const uint32_t rank = blockIdx.x - g.g_base;
@@ -1038,7 +1038,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
         }
         if (s_flag) {
             // reliable update: u += x in FP64, then r = b - A u in FP64
-            const bool judge = sc.judge(a.max_iter);
+            const bool check = sc.may_end(a.max_iter);
             double2* const u = reinterpret_cast<double2*>(a.u);
             for (uint32_t s = s0 + warp; s < s1; s += nw) {
                 const uint32_t i = s * 32 + lane;
@@ -1053,7 +1053,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
             if (sync()) goto done;
             double rrl = 0.0, rpl = 0.0;
             FFAcc rzk{0.f, 0.f};
-            true_residual_ghost<kThreads>(a, r4, P, W, s0, s1, judge, rrl, rzk, nullptr, &rpl);
+            true_residual_ghost<kThreads>(a, r4, P, W, s0, s1, check, rrl, rzk, nullptr, &rpl);
             const FF t = rzk.result();
             double v[3] = {rrl, (double)t.hi + (double)t.lo, rpl};
             group_publish<3>(v, red, part2, rank);
@@ -1062,7 +1062,7 @@ __device__ __forceinline__ void mixed_solve_ghost(const MixArgs& a, const Group&
             group_reduce0<3>(part2, G, tt);
             if (tid == 0) {
                 FF be;
-                s_flag = sc.replaced(tt, judge, a.max_iter, be);
+                s_flag = sc.replaced(tt, check, a.max_iter, be);
                 if (!s_flag) {
                     s_beta[0] = be.hi;
                     s_beta[1] = be.lo;

@@ -124,7 +124,7 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
     __shared__ int s_flag;  // 0 iterate, 1 reliable update, 2 stop
     __shared__ int s_fail;   // a wait for ghosts or records ran out
     __shared__ int s_again;  // the fixed-point sum's status: 1 sum by records, 2 give up
-    __shared__ MixScalars sc;  // thread 0 only, but for judge()
+    __shared__ MixScalars sc;  // thread 0 only, but for may_end()
     const unsigned G = kBatch ? g.g_size : gridDim.x;
     const uint32_t rank = kBatch ? blockIdx.x - g.g_base : blockIdx.x;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -217,9 +217,9 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
     };
     // r = b - A u for this lane's row (row_residual) as float-float, z = r / Aii;
     // |r|^2 in FP64, r.z; |b|^2, r.p
-    auto true_residual = [&](bool judge, double& rr, FFAcc& rz, double* bb, double* rp) {
+    auto true_residual = [&](bool check, double& rr, FFAcc& rz, double* bb, double* rp) {
         if (!live) return;
-        const double2 ri = row_residual(a, s, lane, judge, rr, bb);
+        const double2 ri = row_residual(a, s, lane, check, rr, bb);
         if (rp) *rp = dot_with(ri.x, ri.y, kGhost ? P[li] : as4(p), *rp);
         const FF f0 = ff_from_double(ri.x), f1 = ff_from_double(ri.y);
         r = {make_float2(f0.hi, f1.hi), make_float2(f0.lo, f1.lo)};
@@ -407,7 +407,7 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
         }
         if (s_flag) {
             // reliable update: u += x in FP64, then r = b - A u in FP64
-            const bool judge = sc.judge(a.max_iter);
+            const bool check = sc.may_end(a.max_iter);
             if (live) {
                 if (kXGlobal) x = from4(a.x4[i]);
                 double2 ui = u[i];
@@ -420,7 +420,7 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
             if (sync()) goto done;
             double rrl = 0.0, rpl = 0.0;
             FFAcc rzk{0.f, 0.f};
-            true_residual(judge, rrl, rzk, nullptr, &rpl);
+            true_residual(check, rrl, rzk, nullptr, &rpl);
             const FF t = rzk.result();
             double v[3] = {rrl, (double)t.hi + (double)t.lo, rpl};
             group_publish<3>(v, red, part2, rank);
@@ -429,7 +429,7 @@ __device__ __forceinline__ void slice_solve(const MixArgs& a, const Group& g, co
             group_reduce0<3>(part2, G, tt);
             if (tid == 0) {
                 FF be;
-                s_flag = sc.replaced(tt, judge, a.max_iter, be);
+                s_flag = sc.replaced(tt, check, a.max_iter, be);
                 if (!s_flag) {
                     s_beta[0] = be.hi;
                     s_beta[1] = be.lo;
