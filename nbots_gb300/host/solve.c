@@ -194,6 +194,13 @@ fail:
 	return rc;
 }
 
+/* A kernel takes a vector in place only from where a double may stand (a numpy view
+ * into a byte buffer may start anywhere). */
+static int on_double(const void *p)
+{
+	return (uintptr_t)p % sizeof(double) == 0;
+}
+
 int nbg_solver_multiply(nbg_solver_t *s, const double *in, double *out)
 {
 	if (!s->have_pattern)
@@ -208,8 +215,9 @@ int nbg_solver_multiply(nbg_solver_t *s, const double *in, double *out)
 	 * cudaMemcpyAsync, but the host does not wait for it before it launches
 	 * the product (1M dof 0.152 -> 0.138 ms, 66,306 dof 35 -> 28 us; 4,290
 	 * dof 20.7 against 23.5 us) */
-	const int direct = s->host_direct;
-	int rc = direct && s->N >= 16384 ? nbg_copy_in_f64(s->N, in, s->x, s->stream)
+	const int direct = s->host_direct && on_double(out);
+	int rc = s->host_direct && on_double(in) && s->N >= 16384
+			? nbg_copy_in_f64(s->N, in, s->x, s->stream)
 			: nbg_h2d(s->x, in, 8 * (size_t)s->N, s->stream);
 	if (rc == NBG_OK)
 		rc = nbg_spmv_csr_f64(s->N, s->rp, s->ci, s->val, s->x, direct ? out : s->b,
