@@ -11,7 +11,10 @@ thread_local char g_last_error[256] = "";
 int nbg_cuda_error(cudaError_t e) {
     std::snprintf(g_last_error, sizeof(g_last_error), "%s: %s", cudaGetErrorName(e),
                   cudaGetErrorString(e));
-    if (e == cudaErrorMemoryAllocation) return NBG_ERR_NOMEM;
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();  // not left for the check of a later launch to find
+        return NBG_ERR_NOMEM;
+    }
     return NBG_ERR_CUDA;
 }
 

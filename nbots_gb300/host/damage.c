@@ -69,7 +69,9 @@ static void logf_append(FILE *lf, const char *fmt, ...)
 }
 
 typedef struct {
-	double *du, *res, *r, *r_prev, *norm2, *rws, *gws, *bws;
+	double *du, *res, *r, *r_prev, *norm2, *rws, *gws;
+	void *bws;  /* the inner solver's workspace */
+	size_t bws_bytes;
 	uint32_t *lev_ptr, *lev_rows, n_levels;
 	int have_levels;
 } dmg_ws_t;
@@ -143,9 +145,9 @@ int nbg_fem_damage(nbg_fem_t *f, const nbg_bcs_t *bcs, double E, double nu, doub
 	TRY(nbg_dev_alloc((void **)&w.rws, nbg_residual_workspace_bytes(N) + 8));
 	w.norm2 = w.rws + nbg_residual_workspace_bytes(N) / 8;
 	TRY(nbg_fem_cg_workspace(f));
-	const size_t bws_bytes = nbg_cg_bsr_layout_workspace_bytes(&f->bsr);
 	if (blocked)
-		TRY(nbg_dev_alloc((void **)&w.bws, bws_bytes));
+		TRY(nbg_ws_grow(&w.bws, &w.bws_bytes, nbg_cg_bsr_layout_workspace_bytes(&f->bsr),
+				nbg_cg_bsr_workspace_bytes(N)));
 	Eh = malloc(8 * (size_t)(ne ? ne : 1));
 	rh = malloc(8 * (npt ? npt : 1));
 	if (!Eh || !rh)
@@ -203,7 +205,7 @@ int nbg_fem_damage(nbg_fem_t *f, const nbg_bcs_t *bcs, double E, double nu, doub
 							    ? NBG_CG_JACOBI | NBG_CG_NBOTS_STOP |
 							      NBG_CG_FIXED_ORDER
 							    : NBG_CG_JACOBI,
-						    &cg, w.bws, bws_bytes, f->stream);
+						    &cg, w.bws, w.bws_bytes, f->stream);
 			} else {
 				st = nbg_cg_f64(N, f->row_ptr, f->col_idx, f->K, w.res, w.du, N, 1e-8,
 						NBG_CG_JACOBI, &cg, f->cg_ws, f->cg_ws_bytes, f->stream);

@@ -726,17 +726,13 @@ static int zero_u(nbg_fem_t *f)
 	return nbg_memset(f->u, 0, 8 * (size_t)f->N, f->stream);
 }
 
-static int ensure_ws(nbg_fem_t *f, size_t need)
+/* The workspace of the mixed solver, or of the FP64 block CG. */
+static int ensure_ws(nbg_fem_t *f, int mixed)
 {
-	if (f->cg_ws_bytes >= need)
-		return NBG_OK;
-	nbg_dev_free(f->cg_ws);
-	f->cg_ws = NULL;
-	f->cg_ws_bytes = 0;
-	int rc = nbg_dev_alloc(&f->cg_ws, need);
-	if (rc == NBG_OK)
-		f->cg_ws_bytes = need;
-	return rc;
+	const size_t need = mixed ? nbg_cg_mixed_layout_workspace_bytes(&f->bsr)
+				  : nbg_cg_bsr_layout_workspace_bytes(&f->bsr);
+	return nbg_ws_grow(&f->cg_ws, &f->cg_ws_bytes, need,
+			   mixed ? need : nbg_cg_bsr_workspace_bytes(f->N));
 }
 
 int nbg_fem_solve_fast(nbg_fem_t *f, uint32_t max_iter, double tol, unsigned flags,
@@ -744,7 +740,7 @@ int nbg_fem_solve_fast(nbg_fem_t *f, uint32_t max_iter, double tol, unsigned fla
 {
 	int rc = NBG_OK;
 	TRY(fill_layout(f));
-	TRY(ensure_ws(f, nbg_cg_bsr_layout_workspace_bytes(&f->bsr)));
+	TRY(ensure_ws(f, 0));
 	TRY(zero_u(f));
 	return nbg_cg_bsr_f64(&f->bsr, f->F, f->u, max_iter, tol, flags, res, f->cg_ws,
 			      f->cg_ws_bytes, f->stream);
@@ -757,7 +753,7 @@ int nbg_fem_solve_mixed(nbg_fem_t *f, uint32_t max_iter, double tol, double delt
 {
 	int rc = NBG_OK;
 	TRY(fill_layout(f));
-	TRY(ensure_ws(f, nbg_cg_mixed_layout_workspace_bytes(&f->bsr)));
+	TRY(ensure_ws(f, 1));
 	TRY(zero_u(f));
 	return nbg_cg_mixed(&f->bsr, f->F, f->u, max_iter, tol, delta, flags, res, f->cg_ws,
 			    f->cg_ws_bytes, f->stream);
@@ -850,9 +846,7 @@ static int solve_rhs(nbg_fem_t *f, const double *b, double *x, double tol, int m
 	int rc = fill_layout(f);
 	if (rc != NBG_OK)
 		return rc;
-	const size_t need = method == NBG_METHOD_MIXED ? nbg_cg_mixed_layout_workspace_bytes(&f->bsr)
-						      : nbg_cg_bsr_layout_workspace_bytes(&f->bsr);
-	if ((rc = ensure_ws(f, need)) != NBG_OK)
+	if ((rc = ensure_ws(f, method == NBG_METHOD_MIXED)) != NBG_OK)
 		return rc;
 	if (method == NBG_METHOD_MIXED) {
 		nbg_mixed_result_t r;

@@ -78,6 +78,10 @@ int nbg_fem_pick_nodes(uint32_t n, const uint32_t *ids, const double *nod, doubl
 int nbg_fem_event_ptr(uint32_t N, uint32_t n_ev, const uint32_t *ev_dof, uint32_t *ev_ptr,
 		      void *stream);
 
+/* Grow the device workspace *ws of *have bytes, whose content is lost, to `want` bytes,
+ * or, where there is no memory for them, to `least` (solve.c). */
+int nbg_ws_grow(void **ws, size_t *have, size_t want, size_t least);
+
 /* Grow f's CG workspace to what nbg_cg_f64 needs for f->N dofs. */
 int nbg_fem_cg_workspace(nbg_fem_t *f);
 

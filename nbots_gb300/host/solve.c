@@ -10,7 +10,7 @@
 #include <stdlib.h>
 #include <string.h>
 
-#include "nbots_gb300.h"
+#include "fem_internal.h"
 
 /* csrc/spmv.cu: n doubles of coherent host memory to the device, by a kernel */
 int nbg_copy_in_f64(size_t n, const double *src, double *dst, void *stream);
@@ -135,6 +135,24 @@ fail:
 	return rc;
 }
 
+int nbg_ws_grow(void **ws, size_t *have, size_t want, size_t least)
+{
+	if (*have >= want)
+		return NBG_OK;
+	nbg_dev_free(*ws);
+	*ws = NULL;
+	*have = 0;
+	size_t bytes = want;
+	int rc = nbg_dev_alloc(ws, bytes);
+	if (rc == NBG_ERR_NOMEM && least < want) {
+		bytes = least;
+		rc = nbg_dev_alloc(ws, bytes);
+	}
+	if (rc == NBG_OK)
+		*have = bytes;
+	return rc;
+}
+
 int nbg_solver_solve(nbg_solver_t *s, const double *b, double *x, uint32_t max_iter,
 		     double tol, unsigned flags, int method, nbg_solve_info_t *info)
 {
@@ -148,16 +166,13 @@ int nbg_solver_solve(nbg_solver_t *s, const double *b, double *x, uint32_t max_i
 		method = NBG_METHOD_NBOTS;
 	if (method != NBG_METHOD_NBOTS && !s->bsr_ok)
 		return NBG_ERR_PATTERN;
-	size_t need = method == NBG_METHOD_NBOTS ? nbg_cg_workspace_bytes(s->N)
-		    : method == NBG_METHOD_MIXED ? nbg_cg_mixed_layout_workspace_bytes(&s->bsr)
-		    : nbg_cg_bsr_layout_workspace_bytes(&s->bsr);
-	if (s->ws_bytes < need) {
-		nbg_dev_free(s->ws);
-		s->ws = NULL;
-		s->ws_bytes = 0;
-		TRY(nbg_dev_alloc(&s->ws, need));
-		s->ws_bytes = need;
-	}
+	const size_t need = method == NBG_METHOD_NBOTS ? nbg_cg_workspace_bytes(s->N)
+			  : method == NBG_METHOD_MIXED ? nbg_cg_mixed_layout_workspace_bytes(&s->bsr)
+			  : nbg_cg_bsr_layout_workspace_bytes(&s->bsr);
+	/* the FP64 block CG runs without its plan too */
+	const size_t least = method == NBG_METHOD_NBOTS || method == NBG_METHOD_MIXED
+				   ? need : nbg_cg_bsr_workspace_bytes(s->N);
+	TRY(nbg_ws_grow(&s->ws, &s->ws_bytes, need, least));
 	TRY(nbg_h2d(s->b, b, 8 * (size_t)s->N, s->stream));
 	TRY(nbg_h2d(s->x, x, 8 * (size_t)s->N, s->stream));
 	if (method == NBG_METHOD_MIXED) {
