@@ -411,7 +411,7 @@ int nbg_solver_solve(nbg_solver_t *s, const double *b, double *x, uint32_t max_i
                      double tol, unsigned flags, int method, nbg_solve_info_t *info);
 
 /* y = A x with nbots' row sums (nbg_spmv_csr_f64, bit-exact) on the
- * solver's matrix; in and out in host memory. */
+ * solver's matrix; in and out in host memory, at any address. */
 int nbg_solver_multiply(nbg_solver_t *s, const double *in, double *out);
 /* Device pointers of the solver's CSR (valid until the next set_matrix with a
  * new pattern or destroy); any output may be NULL.  A caller that writes
